@@ -1,0 +1,73 @@
+"""GPU: the warp-column pass pairs (fft_pipe.cuh) against the barrier form of the
+same pairs and against FP64.
+
+Buffers on 16-byte boundaries take the warp-column form once a launch has more
+tiles than resident CTAs; the same rows at an odd multiple of 8 bytes take the
+barrier form.  Both do the same arithmetic: the same bits, except at 2^19 and
+2^20 (scalar against packed butterflies; FP64 bound only).  Batches: the
+smallest that take the form, odd ones, one with several rounds of the ring."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL_REL_L2 = 2e-6
+
+
+@pytest.mark.parametrize("logn,batch", [(15, 20), (15, 301), (16, 11), (16, 203), (17, 5), (17, 67), (18, 3), (18, 33),
+                                        (19, 2), (19, 13), (20, 2), (20, 5), (21, 1), (21, 3), (22, 2), (23, 1),
+                                        (24, 1), (25, 1), (26, 1)])
+def test_pipe_matches_barrier_form_and_fp64(lib_built, logn, batch):
+    import gbfft
+    torch = pytest.importorskip("torch")
+    n = 1 << logn
+    g = torch.Generator(device="cuda")
+    g.manual_seed(700 + logn)
+    x = torch.view_as_complex(torch.randn(batch * n + 1, 2, generator=g, device="cuda"))
+    a = x[1:].clone()  # 16-byte aligned copy of the rows at x + 8 bytes
+    assert a.data_ptr() % 16 == 0 and x.data_ptr() % 16 == 0
+    with gbfft.Context(0) as ctx:
+        for direction in (gbfft.FORWARD, gbfft.INVERSE):
+            y = torch.full_like(a, float("nan"))
+            z = torch.full_like(x, float("nan"))
+            for _ in range(2):  # the second launch finds the counters cleared
+                ctx.c2c_device(a, y, n, batch, direction, stream=torch.cuda.current_stream().cuda_stream)
+            ctx.c2c_device(x.data_ptr() + 8, z.data_ptr() + 8, n, batch, direction,
+                           stream=torch.cuda.current_stream().cuda_stream)
+            torch.cuda.synchronize()
+            if logn not in (19, 20):
+                assert torch.equal(torch.view_as_real(y), torch.view_as_real(z[1:]))
+            assert torch.isnan(z[0].real)
+            for row in {0, batch // 2, batch - 1}:
+                r = a[row * n:(row + 1) * n].to(torch.complex128)
+                want = torch.fft.fft(r) if direction == gbfft.FORWARD else torch.fft.ifft(r)
+                got = y[row * n:(row + 1) * n].to(torch.complex128)
+                assert ((got - want).norm() / want.norm()).item() <= TOL_REL_L2
+        ctx.c2c_host(np.zeros((1, 1 << 15), np.complex64))  # reports a device wait that gave up, if any did
+
+
+def test_pipe_under_capture_and_on_two_streams(lib_built):
+    import gbfft
+    torch = pytest.importorskip("torch")
+    n, batch = 1 << 16, 64
+    xs = [torch.view_as_complex(torch.randn(batch, n, 2, device="cuda")) for _ in range(2)]
+    ys = [torch.empty_like(x) for x in xs]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    with gbfft.Context(0) as ctx:
+        for _ in range(4):
+            for x, y, s in zip(xs, ys, streams):
+                ctx.c2c_device(x, y, n, batch, gbfft.FORWARD, stream=s.cuda_stream)
+        torch.cuda.synchronize()
+        want = [y.clone() for y in ys]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=streams[0]):
+            ctx.c2c_device(xs[0], ys[0], n, batch, gbfft.FORWARD, stream=streams[0].cuda_stream)
+        for _ in range(3):
+            ys[0].zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(torch.view_as_real(ys[0]), torch.view_as_real(want[0]))
+    for x, y in zip(xs, want):
+        ref = torch.fft.fft(x[:2].to(torch.complex128))
+        assert ((y[:2].to(torch.complex128) - ref).norm() / ref.norm()).item() <= TOL_REL_L2

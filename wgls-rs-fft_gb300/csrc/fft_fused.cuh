@@ -212,16 +212,16 @@ __device__ __forceinline__ void fused_loop(const FusedParams &P, float2 *smem_f,
 
 // The last CTA to finish clears the counters for the next launch; every
 // other CTA has published all its work before it counts itself out.
+// flag: a word of shared memory.
 template <int THREADS>
-__device__ __forceinline__ void fused_finish(const FusedParams &P) {
-    __shared__ int s_last;
+__device__ __forceinline__ void fused_finish(const FusedParams &P, int *flag) {
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        s_last = atomicAdd(P.ctr + 1, 1u) == gridDim.x - 1;
+        *flag = atomicAdd(P.ctr + 1, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (s_last) {
+    if (*flag) {
         __threadfence();
         for (uint32_t i = threadIdx.x; i < 2u + P.ngroups; i += THREADS) P.ctr[i] = 0u;
     }
@@ -236,7 +236,8 @@ fft_fused_kernel(FusedParams P) {
     // ones measured faster (2^19: 152.4 against 149.8 GSa/s)
     using Eng = std::conditional_t<(LOGRA >= 10 || LOGRB >= 10), DftRegsScalar, DftRegs>;
     fused_loop<LOGRA, LOGRB, THREADS, LOGN, LOGPA, LE>(P, smem_f, Eng{});
-    fused_finish<THREADS>(P);
+    __shared__ int s_last;
+    fused_finish<THREADS>(P, &s_last);
 }
 
 template <int LOGRA, int LOGRB, int THREADS, int LOGN, int LOGPA, int LE = 4>

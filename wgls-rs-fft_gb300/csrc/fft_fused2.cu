@@ -5,15 +5,17 @@
 
 #include "gbfft_internal.h"
 #include "gbfft_plan.h"
-#include "fft_fused.cuh"
+#include "fft_pipe.cuh"
+#include "tensor_map.h"
 
 namespace gbfft {
 
 bool fused2_kernel_info(int logr1, int logr2, FusedDesc &d, int loge) {
+    pipe2_kernel_info(logr1, logr2, d.pipe, loge);
     if (loge == 5) {
 #define GBFFT_F2E(A, B, T) \
     if (logr1 == A && logr2 == B) { fused_describe<A, B, T, A + B, 0, 5>(d); return true; }
-        GBFFT_F2E(8, 7, 128)
+        GBFFT_F2E(7, 8, 128)
         GBFFT_F2E(8, 8, 128)
         GBFFT_F2E(9, 8, 256)
         GBFFT_F2E(9, 9, 256)
@@ -27,7 +29,7 @@ bool fused2_kernel_info(int logr1, int logr2, FusedDesc &d, int loge) {
     if (logr1 == A && logr2 == B) { fused_describe<A, B, T, A + B, 0>(d); return true; }
     GBFFT_F2(7, 6, 128)
     GBFFT_F2(7, 7, 128)
-    GBFFT_F2(8, 7, 256)
+    GBFFT_F2(7, 8, 256)
     GBFFT_F2(8, 8, 256)
     GBFFT_F2(9, 8, 512)
     GBFFT_F2(9, 9, 512)
@@ -54,6 +56,13 @@ cudaError_t fused_prepare(FusedDesc &d) {
         e = cudaFuncSetAttribute(d.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.smem);
         if (e != cudaSuccess) return e;
     }
+    if (d.pipe.fn) {
+        e = cudaFuncSetAttribute(d.pipe.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.pipe.smem);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.pipe.ctas_per_sm, d.pipe.fn, d.pipe.threads,
+                                                              d.pipe.smem);
+        if (e != cudaSuccess) return e;
+    }
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.ctas_per_sm, d.fn, d.threads, d.smem);
     if (e != cudaSuccess || d.tmem_cols <= 0) return e;
     // Split forms: the occupancy query answers 1 for kernels that allocate
@@ -78,15 +87,29 @@ cudaError_t fused_prepare(FusedDesc &d) {
     return cudaSuccess;
 }
 
-uint32_t fused_lag(const FusedDesc &d, uint64_t ngroups, int sms) {
-    const uint64_t grid = (uint64_t)std::max(1, d.ctas_per_sm) * (uint64_t)std::max(1, sms);
-    const uint64_t per = 2ull * d.tiles_per_group;
+uint32_t fused_lag(uint64_t inflight, uint32_t tiles_per_group, uint64_t group_samples, uint64_t ngroups) {
+    const uint64_t per = 2ull * tiles_per_group;
     // enough queue between producer and consumer that consumers rarely wait
-    uint64_t lag = (2 * grid + per - 1) / per;
+    uint64_t lag = (2 * inflight + per - 1) / per;
     // ... but a window of intermediates that stays well inside L2
-    const uint64_t cap = std::max<uint64_t>(1, kFusedWindowBytes / (8ull * d.group_samples));
+    const uint64_t cap = std::max<uint64_t>(1, kFusedWindowBytes / (8ull * group_samples));
     lag = std::min(std::max<uint64_t>(lag, 1), cap);
     return (uint32_t)std::min<uint64_t>(lag, ngroups);
+}
+
+// 3-D tensor map of float pairs: `cols` complex a row, `rows` rows of stride
+// `cols`, `mats` matrices back to back; boxes of box_cols columns x <= 256 rows.
+static bool pipe_map(CUtensorMap *map, const void *base, uint64_t cols, uint64_t rows, uint64_t mats, int box_cols) {
+    PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    if (!encode) return false;
+    const cuuint64_t dims[3] = {2 * cols, rows, mats};
+    const cuuint64_t strides[2] = {cols * sizeof(float2), rows * cols * sizeof(float2)};
+    const cuuint32_t box[3] = {2u * (cuuint32_t)box_cols, (cuuint32_t)std::min<uint64_t>(rows, 256), 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)base, dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  box_cols == 16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint64_t batch, const float2 *tw_a,
@@ -100,8 +123,6 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
     P.out = out;
     P.batch = (uint32_t)batch;
     P.ngroups = (uint32_t)(batch * d.groups_per_transform);
-    P.lag = fused_lag(d, P.ngroups, sms);
-    P.nitems = 2u * d.tiles_per_group * P.ngroups;
     P.tw_a = tw_a;
     P.tw_b = tw_b;
     P.tw_lo = tw_lo;
@@ -114,8 +135,38 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
     P.err = err;
     P.spin_limit = 1u << 22;  // ~0.5 s of 128 ns polls; a healthy wait is a few microseconds
     P.gtab = (const uint4 *)gtab;
-    const uint64_t grid = std::min<uint64_t>((uint64_t)P.nitems,
-                                             (uint64_t)std::max(1, d.ctas_per_sm) * (uint64_t)std::max(1, sms));
+    // The warp-column form (fft_pipe.cuh) needs tensor maps: buffers on 16-byte
+    // boundaries, and no tables of row addresses.  It is the faster one wherever
+    // its ring of tiles fills (2^16 x 1024: 297 -> 237 us, 2^16 x 32: 21.6 ->
+    // 21.2), but takes longer to start: a launch of no more tiles than resident
+    // CTAs, or of a single group (no second pass can start before the whole first
+    // one is done), is left to the barrier form (2^16 x 4: 12.3 against 10.3 us,
+    // 2^20 x 1: 21.5 against 20.5).  Load options stay with the barrier form, whose
+    // lanes run along the columns: here they run along the rows, and each window
+    // factor would be a sector of its own (2^16 x 1024: 342 against 315 us).
+    const uint64_t pipe_ctas = (uint64_t)d.pipe.ctas_per_sm * (uint64_t)std::max(1, sms);
+    if (d.pipe.fn && !tab_in && !tab_out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && P.ngroups > 1 &&
+        2ull * d.pipe.tiles_per_group * P.ngroups > pipe_ctas && !(d.pipe.first && (ops.win || ops.noise_sigma != 0.f))) {
+        PipeParams Q;
+        const uint64_t n = 1ull << d.logn, ra = 1ull << d.logra, rb = 1ull << d.logrb, p = 1ull << d.logpa;
+        if (pipe_map(&Q.map_in, in, n / ra, ra, batch, d.pipe.box_cols_a) &&
+            pipe_map(&Q.map_mid, out, d.logpa ? p : n / ra, ra, d.logpa ? batch * (n / ra / p) : batch,
+                     d.pipe.box_cols_a) &&
+            pipe_map(&Q.map_io, out, n / rb, rb, batch, d.pipe.box_cols_b)) {
+            P.nitems = 2u * d.pipe.tiles_per_group * P.ngroups;
+            P.lag = fused_lag(pipe_ctas * d.pipe.slots, d.pipe.tiles_per_group, d.group_samples, P.ngroups);
+            Q.fact_a = d.pipe.fact_a;
+            Q.fact_b = d.pipe.fact_b;
+            Q.f = P;
+            void *args[] = {(void *)&Q};
+            return cudaLaunchKernel(d.pipe.fn, dim3((unsigned)std::min<uint64_t>(P.nitems, pipe_ctas)),
+                                    dim3(d.pipe.threads), args, d.pipe.smem, stream);
+        }
+    }
+    const uint64_t ctas = (uint64_t)std::max(1, d.ctas_per_sm) * (uint64_t)std::max(1, sms);
+    P.nitems = 2u * d.tiles_per_group * P.ngroups;
+    P.lag = fused_lag(ctas, d.tiles_per_group, d.group_samples, P.ngroups);
+    const uint64_t grid = std::min<uint64_t>((uint64_t)P.nitems, ctas);
     void *args[] = {(void *)&P};
     return cudaLaunchKernel(d.fn, dim3((unsigned)grid), dim3(d.threads), args, d.smem, stream);
 }

@@ -9,6 +9,7 @@
 namespace gbfft {
 
 bool fused3_kernel_info(int logn, FusedDesc &d) {
+    pipe3_kernel_info(logn, d.pipe);
 #define GBFFT_F3(L) \
     if (logn == L) { fused_describe<8, 8, 256, L, L - 16>(d); return true; }
     GBFFT_F3(21)

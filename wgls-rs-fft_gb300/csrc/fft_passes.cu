@@ -22,14 +22,12 @@
 // The first factor is one lookup per thread; the second depends only on the
 // column and e, so the CTA builds it once into a padded 16 x 17 shared table.
 // Both come from two FP64-built tables (W_N^i for i < 2^s and W_N^{i 2^s}).
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include <algorithm>
 
 #include "gbfft_internal.h"
 #include "gbfft_plan.h"
 #include "fft_tc.cuh"
+#include "tensor_map.h"
 #include "fft_tiles.cuh"
 
 namespace gbfft {
@@ -298,7 +296,7 @@ fft_pass_first_tma_persistent_kernel(const __grid_constant__ CUtensorMap map, fl
 // host side
 // ---------------------------------------------------------------------------
 
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q;

@@ -178,7 +178,8 @@ fft_fused_tc_kernel(FusedParams P) {
         fused_loop<LOGRA, LOGRB, THREADS, LOGN, 0, 5>(P, (float2 *)smem_ftc, DftTc32<KIND>{&st});
     else
         fused_loop<LOGRA, LOGRB, THREADS, LOGN, 0>(P, (float2 *)smem_ftc, DftTc<KIND>{&st});
-    fused_finish<THREADS>(P);
+    __shared__ int s_last;
+    fused_finish<THREADS>(P, &s_last);
     tc_cta_teardown<typename C::L>(st);
 }
 

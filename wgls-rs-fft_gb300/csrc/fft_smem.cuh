@@ -143,14 +143,21 @@ __device__ __forceinline__ float2 twiddle_mul(float2 a, float2 b) {
     else return cmul(a, b);
 }
 
+// Twiddle-table entry; SHARED: the table is a copy in shared memory.
+template <bool SHARED>
+__device__ __forceinline__ float2 ld_tab(const float2 *p) {
+    if constexpr (SHARED) return *p;
+    else return ld_tw(p);
+}
+
 // Butterflies of one sub-pass on the register array v.
-template <int LOGE, int LOGR, int LOGP, int LOGT, bool FACT = false, class Eng = DftRegs>
+template <int LOGE, int LOGR, int LOGP, int LOGT, bool FACT = false, class Eng = DftRegs, bool SHARED = false>
 __device__ __forceinline__ void subpass_compute(float2 (&v)[1 << LOGE], int t, const float2 *tw, Eng &eng) {
     constexpr int E = 1 << LOGE, R = 1 << LOGR, NB = E / R, P = 1 << LOGP, T = 1 << LOGT;
     if constexpr (FACT) {
         float2 wt[R];
 #pragma unroll
-        for (int m = 1; m < R; ++m) wt[m] = ld_tw(tw + (m - 1) * T + t);
+        for (int m = 1; m < R; ++m) wt[m] = ld_tab<SHARED>(tw + (m - 1) * T + t);
         auto body = [&](auto bc) {
             constexpr int b = decltype(bc)::value;
             float2 x[R];
@@ -181,7 +188,7 @@ __device__ __forceinline__ void subpass_compute(float2 (&v)[1 << LOGE], int t, c
                 const int j = t + T * b;
                 const int k = j & (P - 1);
 #pragma unroll
-                for (int m = 1; m < R; ++m) x[m] = twiddle_mul<Eng>(x[m], ld_tw(tw + (m - 1) * P + k));
+                for (int m = 1; m < R; ++m) x[m] = twiddle_mul<Eng>(x[m], ld_tab<SHARED>(tw + (m - 1) * P + k));
             }
             eng.template run<R>(x);
 #pragma unroll
@@ -201,11 +208,11 @@ inline int subcfg_segments(TwiddleSegment *out, uint64_t base) {
 }
 
 // Sub-pass I of the schedule of SubCfg<LOGN, LE> (twiddle table already offset).
-template <int LOGN, int I, int LE = 4, class Eng = DftRegs>
+template <int LOGN, int I, int LE = 4, class Eng = DftRegs, bool SHARED = false>
 __device__ __forceinline__ void subpass_run(float2 (&v)[SubCfg<LOGN, LE>::E], int t, const float2 *tw_all, Eng &eng) {
     using C = SubCfg<LOGN, LE>;
-    subpass_compute<C::LOGE, C::logr(I), C::logp(I), C::LOGT, C::factored(I), Eng>(v, t, tw_all + C::tw_offset(I),
-                                                                                     eng);
+    subpass_compute<C::LOGE, C::logr(I), C::logp(I), C::LOGT, C::factored(I), Eng, SHARED>(
+        v, t, tw_all + C::tw_offset(I), eng);
 }
 
 // Position (within the transform) of output q of butterfly slot b after

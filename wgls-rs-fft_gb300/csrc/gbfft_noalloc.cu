@@ -89,6 +89,7 @@ int na_setup(int dev, cudaStream_t stream, NaDevice &d) {
     uint64_t off = 0;
     for (int L = kNaMinLogN; L <= kNaMaxLogN; ++L) {
         std::vector<int> parts = split_passes(L);
+        pass_order(parts);
         if (parts.size() != 2) return GBFFT_ERR_UNSUPPORTED;
         std::vector<PassDesc> passes(2);
         int logp = 0;

@@ -40,6 +40,7 @@ void DeviceBuffer::release() {
 
 Plan::~Plan() {
     if (tw) cudaFree(tw);
+    if (fact) cudaFree(fact);
     if (gtab) cudaFree(gtab);
 }
 
@@ -51,6 +52,13 @@ std::vector<int> split_passes(int logn, int max_logr) {
     std::vector<int> parts(p, logn / p);
     for (int i = 0; i < logn % p; ++i) parts[i] += 1;
     return parts;
+}
+
+// 2^15 takes 2^7 first: in the fused pair the second pass's tiles carry their
+// inter-pass factors, and with 256 rows (16 columns) those of three slots fit two
+// CTAs an SM beside the tiles; with 128 rows (32 columns) they do not.
+void pass_order(std::vector<int> &parts) {
+    if (parts.size() == 2 && parts[0] == 8 && parts[1] == 7) std::swap(parts[0], parts[1]);
 }
 
 uint64_t multipass_segments(int logn, std::vector<PassDesc> &passes, uint64_t off,
@@ -130,10 +138,11 @@ std::vector<PlanVariant> plan_candidates(int logn, int precision) {
         if (pass_kernel_info(logn - 16, true, pd, 4, 3, true)) c.push_back(PlanVariant{10, false, true, 3, 4, true});
     }
     for (int m = top; m >= 7; --m) {
-        const std::vector<int> parts = split_passes(logn, m);
+        std::vector<int> parts = split_passes(logn, m);
         bool dup = false;
         for (const PlanVariant &v : c) dup |= split_passes(logn, v.max_logr) == parts;
         if (dup || parts[0] < 5) continue;
+        if (!tc) pass_order(parts);
         // the pair with 32 samples a thread (radix-32 sub-passes) first where a
         // pass has radix 2^9 or more: measured faster at 2^17..2^20 (177 / 178.5 /
         // 150.7 / 155.9 against 174.7 / 166.2 / 145.6 / 144.7 GSa/s); after the
@@ -204,6 +213,7 @@ int plan_build(Plan &p, int logn, int precision, const PlanVariant &v, cudaStrea
         // the split form's radix-2^10 tile would not fit in shared memory
         std::vector<int> parts = split_passes(logn, tc ? std::min(9, v.max_logr) : v.max_logr);
         if (small_fused) parts = {7, logn - 7};
+        if (!tc) pass_order(parts);
         const bool fused3 = v.fused && !tc && fused3_kernel_info(logn, p.fused);
         if (fused3) parts = {logn - 16, 8, 8};
         int logp = 0;
@@ -278,6 +288,32 @@ int plan_build(Plan &p, int logn, int precision, const PlanVariant &v, cudaStrea
             why = cudaGetErrorString(e);
             return GBFFT_ERR_CUDA;
         }
+    }
+    PipeDesc &pd = p.fused.pipe;
+    if (p.has_fused && pd.fn) {
+        const int logpa = p.fused.logpa, logpb = logpa + p.fused.logra;
+        const uint64_t na = logpa ? factors_count(p.fused.logra, logpa, pd.loge) : 0;
+        const uint64_t nb = factors_count(p.fused.logrb, logpb, pd.loge);
+        if (cudaMalloc(&p.fact, (na + nb) * sizeof(float4)) != cudaSuccess) {
+            cudaGetLastError();  // no room (64 MB at 2^26): the barrier form needs no factor table
+            p.fact = nullptr;
+            pd.fn = nullptr;
+            return GBFFT_OK;
+        }
+        const float2 *lo = p.tw + p.tw_lo_offset, *hi = p.tw + p.tw_hi_offset;
+        e = cudaSuccess;
+        if (na)
+            e = factors_fill(p.fact, lo, hi, p.tw_split, logn, p.fused.logra, logpa, pd.loge, pd.logtile, pd.soa,
+                             stream);
+        if (e == cudaSuccess)
+            e = factors_fill(p.fact + na, lo, hi, p.tw_split, logn, p.fused.logrb, logpb, pd.loge, pd.logtile, pd.soa,
+                             stream);
+        if (e != cudaSuccess) {
+            why = cudaGetErrorString(e);
+            return GBFFT_ERR_CUDA;
+        }
+        pd.fact_a = p.fact;
+        pd.fact_b = p.fact + na;
     }
     return GBFFT_OK;
 }

@@ -44,7 +44,25 @@ struct PassDesc {
 // first pass's tiles of group x with the second pass's tiles of group x - LAG,
 // so that the intermediate is read back from L2 (fft_fused.cuh): both passes
 // of a two-pass transform, or the last two of a three-pass one.
+//
+// PipeDesc: the same pair with its tiles moved by the tensor memory
+// accelerator and every column inside one warp (fft_pipe.cuh).
+struct PipeDesc {
+    const void *fn = nullptr;
+    int threads = 0;
+    size_t smem = 0;
+    int slots = 0;        // tiles a CTA has in flight
+    int ctas_per_sm = 0;
+    uint32_t tiles_per_group = 0;
+    int box_cols_a = 0, box_cols_b = 0;  // columns of a tensor-map box of either pass
+    bool first = false;                  // pass A is the transform's first pass
+    int loge = 0, logtile = 0;           // log2 of the samples a column and thread / a tile
+    bool soa = false;                    // layout of a factor pair (factors_fill)
+    // inter-pass factors of pass A (three passes only) and B (device, the plan's)
+    const float4 *fact_a = nullptr, *fact_b = nullptr;
+};
 struct FusedDesc {
+    PipeDesc pipe;
     const void *fn = nullptr;
     int threads = 0;
     size_t smem = 0;
@@ -105,6 +123,7 @@ struct Plan {
     // twiddle table (device): rows sub-pass tables, or for multi-pass the
     // per-pass sub-pass tables followed by the two-level W_N table.
     float2 *tw = nullptr;
+    float4 *fact = nullptr;  // inter-pass factors of a warp-column pass pair
     uint64_t tw_entries = 0;
     uint64_t tw_lo_offset = 0, tw_hi_offset = 0;  // W_N^i (i < 2^s), W_N^{i 2^s}
     int tw_split = 0;                             // s
@@ -150,7 +169,19 @@ bool fused2_kernel_info(int logr1, int logr2, FusedDesc &d, int loge = 4);
 int pass_sub_segments(int logr, int loge, TwiddleSegment *out, uint64_t base, int &entries);
 bool fused3_kernel_info(int logn, FusedDesc &d);  // passes 2-3 of (logn - 16, 8, 8)
 cudaError_t fused_prepare(FusedDesc &d);
-uint32_t fused_lag(const FusedDesc &d, uint64_t ngroups, int sms);
+// fft_pipe2.cu, fft_pipe3.cu
+// Inter-pass factors of a global pass of radix 2^logr over p = 2^logp columns,
+// as its tiles of 2^(logtile - logr) columns read them: per tile, two columns a
+// float4 (soa: re, re', im, im'; else re, im, re', im'), W_{R p}^{k T e} for
+// [column pair][e], then W_{R p}^{k t} for [column pair][t], from the plan's
+// two-level table.
+uint64_t factors_count(int logr, int logp, int loge);  // float4 entries
+cudaError_t factors_fill(float4 *out, const float2 *lo, const float2 *hi, int split, int logn, int logr, int logp,
+                         int loge, int logtile, bool soa, cudaStream_t stream);
+bool pipe2_kernel_info(int logr1, int logr2, PipeDesc &d, int loge);
+bool pipe3_kernel_info(int logn, PipeDesc &d);
+// inflight: tiles that the launch's CTAs hold at once
+uint32_t fused_lag(uint64_t inflight, uint32_t tiles_per_group, uint64_t group_samples, uint64_t ngroups);
 cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint64_t batch, const float2 *tw_a,
                          const float2 *tw_b, const float2 *tw_lo, const float2 *tw_hi, float in_im, float out_re,
                          float out_im, LoadOps ops, uint32_t *ctr, uint32_t *err, int sms, cudaStream_t stream,
@@ -158,8 +189,9 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
                          const uint64_t *tab_out = nullptr);
 
 // log2 radices (each <= max_logr) of the global passes for a multi-pass
-// transform of 2^logn.
+// transform of 2^logn, and the order in which the FP32 form takes them.
 std::vector<int> split_passes(int logn, int max_logr = 10);
+void pass_order(std::vector<int> &parts);
 
 // Append the twiddle segments of a multi-pass schedule (per-pass sub-pass
 // tables, then the two-level W_N table) starting at `offset`; fills the pass

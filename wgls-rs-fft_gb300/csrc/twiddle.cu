@@ -4,6 +4,8 @@
 // kept in FP64.  The reference builds its table on the host from an f32 angle
 // (larsjoost/wgls-rs-fft src/lib.rs:761-769), whose rounding reaches ~ulp(2 pi).
 #include "gbfft_internal.h"
+#include "gbfft_plan.h"
+#include "fft_tiles.cuh"
 
 namespace gbfft {
 
@@ -57,6 +59,42 @@ cudaError_t twiddle_fill(float2 *table, const TwiddleSegment *segs, int nseg, cu
     const unsigned threads = 256;
     const uint64_t blocks = (total + threads - 1) / threads;
     twiddle_fill_kernel<<<(unsigned)blocks, threads, 0, stream>>>(table, list, total);
+    return cudaGetLastError();
+}
+
+// Inter-pass factors of a warp-column pass (gbfft_plan.h), one float4 a thread:
+// products of the two-level table's entries, as every other form of the pass
+// computes them, so that all forms give the same bits.
+__global__ void factors_fill_kernel(float4 *out, const float2 *__restrict__ lo, const float2 *__restrict__ hi,
+                                    int split, int logn, int logr, int logp, int loge, int logtile, int soa,
+                                    uint64_t total) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    const int logt = logr - loge, E = 1 << loge, T = 1 << logt;
+    const uint32_t pairs = 1u << (logtile - logr - 1);  // column pairs of a tile
+    const uint32_t per = pairs * (uint32_t)(E + T);
+    const uint64_t tile = i / per;
+    uint32_t r = (uint32_t)(i % per);
+    const bool f = r < pairs * (uint32_t)E;
+    if (!f) r -= pairs * (uint32_t)E;
+    const uint32_t k = 2 * ((uint32_t)tile * pairs + (f ? r >> loge : r >> logt));
+    // W_{R p}^{k T e} or W_{R p}^{k t} as a power of W_N
+    const uint32_t m = f ? r & (uint32_t)(E - 1) : r & (uint32_t)(T - 1);
+    const int sh = logn - logp - (f ? loge : logr);
+    const float2 a = twiddle_2level(lo, hi, (k * m) << sh, split);
+    const float2 b = twiddle_2level(lo, hi, ((k + 1) * m) << sh, split);
+    out[i] = soa ? make_float4(a.x, b.x, a.y, b.y) : make_float4(a.x, a.y, b.x, b.y);
+}
+
+uint64_t factors_count(int logr, int logp, int loge) {
+    return ((uint64_t)((1 << loge) + (1 << (logr - loge))) << logp) / 2;
+}
+
+cudaError_t factors_fill(float4 *out, const float2 *lo, const float2 *hi, int split, int logn, int logr, int logp,
+                         int loge, int logtile, bool soa, cudaStream_t stream) {
+    const uint64_t total = factors_count(logr, logp, loge);
+    factors_fill_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(out, lo, hi, split, logn, logr, logp,
+                                                                            loge, logtile, soa ? 1 : 0, total);
     return cudaGetLastError();
 }
 
