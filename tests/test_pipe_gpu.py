@@ -3,8 +3,7 @@ same pairs and against FP64.
 
 Buffers on 16-byte boundaries take the warp-column form once a launch has more
 tiles than resident CTAs; the same rows at an odd multiple of 8 bytes take the
-barrier form.  Both do the same arithmetic: the same bits, except at 2^19 and
-2^20 (scalar against packed butterflies; FP64 bound only).  Batches: the
+barrier form.  Both do the same arithmetic: the same bits.  Batches: the
 smallest that take the form, odd ones, one with several rounds of the ring."""
 import numpy as np
 import pytest
@@ -35,8 +34,7 @@ def test_pipe_matches_barrier_form_and_fp64(lib_built, logn, batch):
             ctx.c2c_device(x.data_ptr() + 8, z.data_ptr() + 8, n, batch, direction,
                            stream=torch.cuda.current_stream().cuda_stream)
             torch.cuda.synchronize()
-            if logn not in (19, 20):
-                assert torch.equal(torch.view_as_real(y), torch.view_as_real(z[1:]))
+            assert torch.equal(torch.view_as_real(y), torch.view_as_real(z[1:]))
             assert torch.isnan(z[0].real)
             for row in {0, batch // 2, batch - 1}:
                 r = a[row * n:(row + 1) * n].to(torch.complex128)

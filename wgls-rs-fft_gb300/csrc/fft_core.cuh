@@ -76,13 +76,22 @@ constexpr float kSqrtHalf = 0.70710678118654752440f;
 constexpr float kCos1_16 = 0.92387953251128675613f;  // cos(pi/8)
 constexpr float kSin1_16 = 0.38268343236508977173f;  // sin(pi/8)
 
+// A product that is rounded: never contracted into an FMA with the addition that
+// uses it, so that scalar and packed butterflies give the same bits.
+GBFFT_HD float mul_rounded(float a, float b) {
+#if defined(__CUDA_ARCH__)
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
 // a * e^{-i pi/4} = a * (1 - i)/sqrt2
 GBFFT_HD float2 mul_w8_1(float2 a) {
-    return make_float2((a.x + a.y) * kSqrtHalf, (a.y - a.x) * kSqrtHalf);
+    return make_float2(mul_rounded(a.x + a.y, kSqrtHalf), mul_rounded(a.y - a.x, kSqrtHalf));
 }
 // a * e^{-3 i pi/4} = a * (-1 - i)/sqrt2
 GBFFT_HD float2 mul_w8_3(float2 a) {
-    return make_float2((a.y - a.x) * kSqrtHalf, -(a.x + a.y) * kSqrtHalf);
+    return make_float2(mul_rounded(a.y - a.x, kSqrtHalf), -mul_rounded(a.x + a.y, kSqrtHalf));
 }
 // a * e^{-i pi/8}
 GBFFT_HD float2 mul_w16_1(float2 a) {

@@ -213,8 +213,7 @@ struct PairTile : WarpTile<LOGR, LOGTILE, 4> {
 
 // One column a thread, 32 samples.  Packed butterflies for every radix (scalar
 // ones, as the barrier form runs pairs with a radix-2^10 pass: 2^19 288 against
-// 274 us, 2^20 351 against 324), so at 2^19 and 2^20 the two forms may differ in
-// the last bit: the compiler contracts the scalar products into FMAs.
+// 274 us, 2^20 351 against 324; same bits).
 template <int LOGR, int LOGTILE>
 struct ColTile : WarpTile<LOGR, LOGTILE, 5> {
     using B = WarpTile<LOGR, LOGTILE, 5>;
