@@ -1,0 +1,8 @@
+// Single-pass split form, one operand kind (fft_rows_tc.cuh).
+#include "fft_rows_tc.cuh"
+
+namespace gbfft {
+
+template bool rows_tc_info_kind<kTcBF16X6>(int logn, RowsKernelInfo &k);
+
+}  // namespace gbfft

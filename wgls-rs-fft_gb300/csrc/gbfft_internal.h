@@ -41,6 +41,10 @@ struct RowsKernelInfo {
     const void *fn_tab = nullptr;         // forward / inverse over per-row address tables
     const void *fn_tab_inv = nullptr;
     int persist_ctas_per_sm = 0;          // resident CTAs of fn_persistent (set by rows_prepare)
+    // split forms: the tile loop's own shape (the FP32 loop shares the one-shot's)
+    int persist_threads = 0;
+    int persist_transforms = 1;
+    size_t persist_smem = 0;
     int threads = 0;
     int transforms_per_cta = 0;
     size_t smem = 0;

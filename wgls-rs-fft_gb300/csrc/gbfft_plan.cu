@@ -411,7 +411,7 @@ int plan_execute(const Plan &p, const float2 *in, float2 *out, uint64_t batch, i
     }
     if (!p.multipass) {
         e = p.precision != GBFFT_PREC_FP32
-                ? rows_tc_launch(p.rows, in, out, batch, p.tw, direction, p.logn, p.gtab, err, stream, ops)
+                ? rows_tc_launch(p.rows, in, out, batch, p.tw, direction, p.logn, p.gtab, err, p.sms, stream, ops)
                 : rows_launch(p.rows, in, out, batch, p.tw, direction, p.logn, p.variant.persistent, p.sms, stream,
                               ops);
         if (e != cudaSuccess) {

@@ -155,7 +155,7 @@ cudaError_t tc_gtab_fill(void *out, cudaStream_t stream);
 bool rows_tc_kernel_info(int logn, int precision, RowsKernelInfo &k);
 cudaError_t rows_tc_prepare(RowsKernelInfo &k);
 cudaError_t rows_tc_launch(const RowsKernelInfo &k, const float2 *in, float2 *out, uint64_t batch,
-                           const float2 *tw, int direction, int logn, const void *gtab, uint32_t *err,
+                           const float2 *tw, int direction, int logn, const void *gtab, uint32_t *err, int sms,
                            cudaStream_t stream, LoadOps ops);
 // G table: radix 16: [FP16 hi | FP16 lo | BF16 hi | BF16 lo] (2 KB each), [TF32 hi | TF32 lo]
 // (4 KB each); radix 32: [FP16 hi | FP16 lo | BF16 hi | BF16 lo] (8 KB each)
