@@ -25,10 +25,11 @@ def test_warp_tiles(tmp_path):
     out = subprocess.run([exe], capture_output=True, text=True, check=True).stdout.splitlines()
     tiles = [tuple(int(v) for v in line.split()[1:]) for line in out if line.startswith("tile ")]
     dfts = [tuple(int(v) for v in line.split()[1:]) for line in out if line.startswith("dft ")]
-    assert len(tiles) == 5 and len(dfts) == 4
+    assert len(tiles) == 7 and len(dfts) == 4
     for kind, logr, logtile, ok, conflicts in tiles:
         assert ok == 1, (kind, logr, logtile)
-        # a radix-2^10 column fills a warp, which then reads one half of every chunk
-        assert conflicts == (2 if logr == 10 else 1), (kind, logr, conflicts)
+        # one column a thread: a radix-2^10 column fills a warp, which then reads one half
+        # of every chunk
+        assert conflicts == (2 if kind == 5 and logr == 10 else 1), (kind, logr, conflicts)
     for radix, ok in dfts:
         assert ok == 1, radix

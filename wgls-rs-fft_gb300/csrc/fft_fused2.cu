@@ -44,10 +44,15 @@ int pass_sub_segments(int logr, int loge, TwiddleSegment *out, uint64_t base, in
 #define GBFFT_SEG(E, R) \
     case E * 16 + R: entries = SubCfg<R, E>::tw_entries(); return subcfg_segments<R, E>(out, base);
         GBFFT_SEG(5, 7) GBFFT_SEG(5, 8) GBFFT_SEG(5, 9) GBFFT_SEG(5, 10)
-        GBFFT_SEG(4, 5) GBFFT_SEG(4, 6) GBFFT_SEG(4, 7) GBFFT_SEG(4, 8) GBFFT_SEG(4, 9) GBFFT_SEG(4, 10)
+        GBFFT_SEG(4, 11) GBFFT_SEG(4, 5) GBFFT_SEG(4, 6) GBFFT_SEG(4, 7) GBFFT_SEG(4, 8) GBFFT_SEG(4, 9) GBFFT_SEG(4, 10)
 #undef GBFFT_SEG
         default: entries = 0; return -1;
     }
+}
+
+bool wide_usable(const float2 *in, const float2 *out, const LoadOps &ops) {
+    return in != out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && !ops.win && ops.noise_sigma == 0.f &&
+           tensor_map_encoder() != nullptr;
 }
 
 cudaError_t fused_prepare(FusedDesc &d) {
@@ -63,6 +68,7 @@ cudaError_t fused_prepare(FusedDesc &d) {
                                                               d.pipe.smem);
         if (e != cudaSuccess) return e;
     }
+    if (!d.fn) return e;  // the wide two-pass launch has no barrier form
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.ctas_per_sm, d.fn, d.threads, d.smem);
     if (e != cudaSuccess || d.tmem_cols <= 0) return e;
     // Split forms: the occupancy query answers 1 for kernels that allocate
@@ -108,8 +114,13 @@ static bool pipe_map(CUtensorMap *map, const void *base, uint64_t cols, uint64_t
     const cuuint32_t estr[3] = {1, 1, 1};
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)base, dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  box_cols == 16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+                  box_cols == 16  ? CU_TENSOR_MAP_SWIZZLE_128B
+                  : box_cols == 8 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                  : CU_TENSOR_MAP_SWIZZLE_32B,
+                  // 32-byte rows: fetch 64 bytes, the neighbouring tile's share (2^22 x 16: 346
+                  // us; 32, 128 and 256 bytes 359, 359, 363)
+                  box_cols >= 8 ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B : CU_TENSOR_MAP_L2_PROMOTION_L2_64B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint64_t batch, const float2 *tw_a,
@@ -145,8 +156,9 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
     // lanes run along the columns: here they run along the rows, and each window
     // factor would be a sector of its own (2^16 x 1024: 342 against 315 us).
     const uint64_t pipe_ctas = (uint64_t)d.pipe.ctas_per_sm * (uint64_t)std::max(1, sms);
-    if (d.pipe.fn && !tab_in && !tab_out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && P.ngroups > 1 &&
-        2ull * d.pipe.tiles_per_group * P.ngroups > pipe_ctas && !(d.pipe.first && (ops.win || ops.noise_sigma != 0.f))) {
+    const bool filled = P.ngroups > 1 && 2ull * d.pipe.tiles_per_group * P.ngroups > pipe_ctas;
+    if (d.pipe.fn && !tab_in && !tab_out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && (filled || !d.fn) &&
+        !(d.pipe.first && (ops.win || ops.noise_sigma != 0.f))) {
         PipeParams Q;
         const uint64_t n = 1ull << d.logn, ra = 1ull << d.logra, rb = 1ull << d.logrb, p = 1ull << d.logpa;
         if (pipe_map(&Q.map_in, in, n / ra, ra, batch, d.pipe.box_cols_a) &&
@@ -163,6 +175,7 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
                                     dim3(d.pipe.threads), args, d.pipe.smem, stream);
         }
     }
+    if (!d.fn) return cudaErrorInvalidValue;
     const uint64_t ctas = (uint64_t)std::max(1, d.ctas_per_sm) * (uint64_t)std::max(1, sms);
     P.nitems = 2u * d.tiles_per_group * P.ngroups;
     P.lag = fused_lag(ctas, d.tiles_per_group, d.group_samples, P.ngroups);

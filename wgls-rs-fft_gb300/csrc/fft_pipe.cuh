@@ -43,11 +43,14 @@ template <int LOGR, int LOGTILE, int LE> struct PipeTileOf;
 template <int LOGR, int LOGTILE> struct PipeTileOf<LOGR, LOGTILE, 4> { using type = PairTile<LOGR, LOGTILE>; };
 template <int LOGR, int LOGTILE> struct PipeTileOf<LOGR, LOGTILE, 5> { using type = ColTile<LOGR, LOGTILE>; };
 
+template <int LOGR, int LOGTILE> struct PipeTileOf<LOGR, LOGTILE, 6> { using type = WideTile<LOGR, LOGTILE>; };
+
 template <int LOGRA, int LOGRB, int LOGN, int LOGPA, int LE>
 struct PipeCfg {
     // LE 4 (pair tiles): 32 KB tiles, two groups of 4 warps on three slots, two
-    // CTAs an SM.  LE 5: 64 KB tiles (a radix-2^10 tile of 8 columns), two
-    // groups of 8 warps on three slots, one CTA an SM.
+    // CTAs an SM.  LE 5 (one column a thread): 64 KB tiles (a radix-2^10 tile of 8
+    // columns), two groups of 8 warps on three slots, one CTA an SM; LE 6 (wide
+    // tiles, radix 2^10 and 2^11): the same.
     static constexpr int LOGTILE = LE == 4 ? 12 : 13;
     static constexpr int GROUPS = 2, SLOTS = 3;
     static constexpr int WPG = LE == 4 ? 4 : 8;  // warps a group
@@ -151,6 +154,20 @@ __device__ __forceinline__ bool pipe_wait(uint64_t *bar, uint32_t parity, volati
     for (uint32_t polls = 0; !mbar_try_wait(bar, parity);)
         if (*abort || ++polls > kPipeBarSpin) return false;
     return true;
+}
+
+// Whether `ok` holds for all `threads` threads that meet at named barrier `id`.
+__device__ __forceinline__ bool group_all(int id, int threads, bool ok) {
+    uint32_t all;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 q, %3, 0;\n\t"
+        "bar.red.and.pred p, %1, %2, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(all)
+        : "r"(id), "r"(threads), "r"((uint32_t)ok)
+        : "memory");
+    return all != 0;
 }
 
 // Boxes of a tile: at most 256 rows of BOXC columns each.
@@ -309,7 +326,7 @@ __device__ __forceinline__ void pipe_storer(const PipeParams &P, uint8_t *smem, 
 // Pass-A or pass-B work of one warp on a landed tile.
 template <class C, int LOGN, int LOGPA, bool IS_A>
 __device__ __forceinline__ void pipe_compute(const FusedParams &F, uint8_t *smem, uint32_t s, uint32_t grp,
-                                             uint32_t tile, int warp, int lane, uint64_t *free) {
+                                             uint32_t tile, int group, int warp, int lane, uint64_t *free) {
     using K = std::conditional_t<IS_A, typename C::KA, typename C::KB>;
     constexpr bool FIRST = IS_A && C::FIRST_A;
     const uint32_t b = grp / C::GPT, g = grp % C::GPT;
@@ -326,7 +343,7 @@ __device__ __forceinline__ void pipe_compute(const FusedParams &F, uint8_t *smem
             K::twiddle((const float4 *)(smem + C::OFF_TW + s * C::TW_BYTES), t, c, x);
         }
     };
-    K::run(slot, t, c, sub, v, pre, [&] {
+    K::run(slot, t, c, sub, v, group, pre, [&] {
         if constexpr (FIRST) {
             fence_proxy_async_smem();  // this lane's accesses of the slot before the TMA's
             __syncwarp();
@@ -337,7 +354,7 @@ __device__ __forceinline__ void pipe_compute(const FusedParams &F, uint8_t *smem
         K::store_columns(F.out + ((uint64_t)b << LOGN) + ((uint64_t)(col0 + c) << (K::S::LOGT + K::LE)), t, v, l2_evict_last());
     } else {
         if (!IS_A && (F.out_re != 1.0f || F.out_im != 1.0f)) K::scale(v, F.out_re, F.out_im);
-        K::stage(slot, t, c, v);
+        K::stage(slot, t, c, v, group);
     }
 }
 
@@ -370,10 +387,14 @@ fft_pipe_kernel(const __grid_constant__ PipeParams P) {
     } else if (warp == C::COMPUTE + 1) {
         if (lane == 0) pipe_storer<C, LOGN, LOGPA>(P, smem_pipe, B);
     } else {
-        const int wg = warp % C::WPG;
-        for (uint32_t i = (uint32_t)warp / C::WPG;; i += C::GROUPS) {
+        const int wg = warp % C::WPG, cg = warp / C::WPG;
+        for (uint32_t i = (uint32_t)cg;; i += C::GROUPS) {
             const uint32_t s = i % S;
-            if (!__all_sync(0xffffffffu, pipe_wait(B.full + i % D, (i / D) & 1u, B.abort))) {
+            bool ok = __all_sync(0xffffffffu, pipe_wait(B.full + i % D, (i / D) & 1u, B.abort));
+            // warps that share named barriers go on or leave together (names 9, 10; 1 .. 8
+            // are the column pairs')
+            if constexpr (LE == 6) ok = group_all(9 + cg, C::WPG * 32, ok);
+            if (!ok) {
                 if (lane == 0) {
                     *B.abort = 1;
                     atomicExch(P.f.err, 1u);
@@ -385,8 +406,8 @@ fft_pipe_kernel(const __grid_constant__ PipeParams P) {
                 bool is_a;
                 uint32_t grp, tile;
                 fused_item<C::T>(P.f, idx, is_a, grp, tile);
-                if (is_a) pipe_compute<C, LOGN, LOGPA, true>(P.f, smem_pipe, s, grp, tile, wg, lane, B.free + s);
-                else pipe_compute<C, LOGN, LOGPA, false>(P.f, smem_pipe, s, grp, tile, wg, lane, B.free + s);
+                if (is_a) pipe_compute<C, LOGN, LOGPA, true>(P.f, smem_pipe, s, grp, tile, cg, wg, lane, B.free + s);
+                else pipe_compute<C, LOGN, LOGPA, false>(P.f, smem_pipe, s, grp, tile, cg, wg, lane, B.free + s);
                 fence_proxy_async_smem();  // this lane's accesses of the slot before the TMA's
             }
             __syncwarp();
@@ -409,7 +430,7 @@ inline void pipe_describe(PipeDesc &d) {
     d.ctas_per_sm = C::MINB;
     d.tiles_per_group = C::T;
     d.first = C::FIRST_A;
-    d.loge = LE;
+    d.loge = C::KA::LE;
     d.logtile = C::LOGTILE;
     d.soa = C::KA::SOA;
     d.box_cols_a = C::KA::BOXC;

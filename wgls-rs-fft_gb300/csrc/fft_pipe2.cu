@@ -16,4 +16,18 @@ bool pipe2_kernel_info(int logr1, int logr2, PipeDesc &d, int loge) {
     return false;
 }
 
+bool pipe_wide_info(int logn, FusedDesc &d) {
+    switch (logn) {
+        case 21: pipe_describe<11, 10, 21, 0, 6>(d.pipe); break;
+        case 22: pipe_describe<11, 11, 22, 0, 6>(d.pipe); break;
+        default: return false;
+    }
+    d.logra = 11;
+    d.logrb = logn - 11;
+    d.logn = logn;
+    d.groups_per_transform = 1;
+    d.group_samples = 1ull << logn;
+    return true;
+}
+
 }  // namespace gbfft

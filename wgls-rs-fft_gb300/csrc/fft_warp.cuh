@@ -37,18 +37,20 @@ __device__ __forceinline__ void st_policy(float2 *p, float2 v, uint64_t policy) 
 }
 
 // Byte offset, in the tile, of (row, 16-byte chunk) as the TMA's swizzle lays
-// it out: boxes of BOXC columns (128- or 64-byte rows) follow one another.
+// it out: boxes of BOXC columns (128-, 64- or 32-byte rows) follow one another.
 template <int LOGR, int BOXC>
 GBFFT_HD uint32_t warp_tile_off(uint32_t row, uint32_t chunk) {
     if constexpr (BOXC == 16)
         return ((chunk >> 3) << (LOGR + 7)) + (row << 7) + (((chunk & 7) ^ (row & 7)) << 4);
-    else
+    else if constexpr (BOXC == 8)
         return (row << 6) + ((chunk ^ ((row >> 1) & 3)) << 4);
+    else
+        return (row << 5) + ((chunk ^ ((row >> 2) & 1)) << 4);
 }
 // Change of warp_tile_off when the row's low three bits are XORed with i.
 template <int BOXC>
 GBFFT_HD constexpr uint32_t warp_xor(uint32_t i) {
-    return BOXC == 16 ? ((i << 7) | (i << 4)) : ((i << 6) | ((i >> 1) << 4));
+    return BOXC == 16 ? ((i << 7) | (i << 4)) : (BOXC == 8 ? ((i << 6) | ((i >> 1) << 4)) : ((i << 5) | ((i >> 2) << 4)));
 }
 // Row that holds element `pos` of a column between the sub-passes: its low
 // three bits XOR those of pos >> LE, so that the stride-E writes of 8
@@ -71,6 +73,31 @@ struct WarpTile {
     // (two columns) each
     static constexpr int TW_BYTES = COLS * (E + T) * (int)sizeof(float2);
 };
+
+// A last sub-pass of radix R1 < 16: 16 / R1 butterflies, butterfly b's twiddles
+// wt[m] * W_16^{m b}.
+template <int R1>
+__device__ __forceinline__ void pair_factored(const Pair (&wt)[R1], Pair (&x)[16]) {
+    constexpr int NB = 16 / R1;
+    auto body = [&](auto bc) {
+        constexpr int b = decltype(bc)::value;
+        Pair y[R1];
+        y[0] = x[b];
+        auto apply = [&](auto mc) {
+            constexpr int M = decltype(mc)::value + 1;
+            y[M] = pair_mul(pair_mul_w16c<(M * b) & 15>(x[b + M * NB]), wt[M]);
+        };
+        [&]<int... Ms>(std::integer_sequence<int, Ms...>) {
+            (apply(std::integral_constant<int, Ms>{}), ...);
+        }(std::make_integer_sequence<int, R1 - 1>{});
+        PairDft<R1>::run(y);
+#pragma unroll
+        for (int q = 0; q < R1; ++q) x[b + q * NB] = y[q];
+    };
+    [&]<int... Bs>(std::integer_sequence<int, Bs...>) {
+        (body(std::integral_constant<int, Bs>{}), ...);
+    }(std::make_integer_sequence<int, NB>{});
+}
 
 // Two columns a thread, 16 samples of each.
 template <int LOGR, int LOGTILE>
@@ -100,7 +127,7 @@ struct PairTile : WarpTile<LOGR, LOGTILE, 4> {
     // `read` is called after the last read of the tile.
     template <class Pre, class Read>
     __device__ __forceinline__ static void run(uint8_t *tile, int t, int c, const uint8_t *sub, Pair (&x)[E],
-                                               Pre pre, Read read) {
+                                               int, Pre pre, Read read) {
         const uint32_t off0 = warp_tile_off<LOGR, B::BOXC>((uint32_t)t, (uint32_t)c >> 1);
 #pragma unroll
         for (int e = 0; e < E; ++e) {
@@ -123,45 +150,17 @@ struct PairTile : WarpTile<LOGR, LOGTILE, 4> {
             x[e] = Pair{make_float2(q.x, q.y), make_float2(q.z, q.w)};
         }
         read();
-        sub1(t, sub, x);
-    }
-    // sub-pass 1: radix R / 16, NB = 256 / R butterflies
-    __device__ __forceinline__ static void sub1(int t, const uint8_t *sub, Pair (&x)[E]) {
-        constexpr int R1 = 1 << S::logr(1), NB = E / R1, P = 1 << S::tw_logp(1);
         const float4 *tw = (const float4 *)sub + t;
-        if constexpr (NB == 1) {
+        constexpr int R1 = 1 << S::logr(1), P = 1 << S::tw_logp(1);
+        Pair wt[R1];
 #pragma unroll
-            for (int m = 1; m < R1; ++m) {
-                const float4 w = tw[(m - 1) * P];
-                x[m] = pair_mul(x[m], Pair{make_float2(w.x, w.y), make_float2(w.z, w.w)});
-            }
-            PairDft<R1>::run(x);
-        } else {
-            Pair wt[R1];
-#pragma unroll
-            for (int m = 1; m < R1; ++m) {
-                const float4 w = tw[(m - 1) * P];
-                wt[m] = Pair{make_float2(w.x, w.y), make_float2(w.z, w.w)};
-            }
-            auto body = [&](auto bc) {
-                constexpr int b = decltype(bc)::value;
-                Pair y[R1];
-                y[0] = x[b];
-                auto apply = [&](auto mc) {
-                    constexpr int M = decltype(mc)::value + 1;
-                    y[M] = pair_mul(pair_mul_w16c<(M * b) & 15>(x[b + M * NB]), wt[M]);
-                };
-                [&]<int... Ms>(std::integer_sequence<int, Ms...>) {
-                    (apply(std::integral_constant<int, Ms>{}), ...);
-                }(std::make_integer_sequence<int, R1 - 1>{});
-                PairDft<R1>::run(y);
-#pragma unroll
-                for (int q = 0; q < R1; ++q) x[b + q * NB] = y[q];
-            };
-            [&]<int... Bs>(std::integer_sequence<int, Bs...>) {
-                (body(std::integral_constant<int, Bs>{}), ...);
-            }(std::make_integer_sequence<int, NB>{});
+        for (int m = 1; m < R1; ++m) {
+            const float4 w = tw[(m - 1) * P];
+            wt[m] = Pair{make_float2(w.x, w.y), make_float2(w.z, w.w)};
+            if constexpr (R1 == 16) x[m] = pair_mul(x[m], wt[m]);
         }
+        if constexpr (R1 == 16) PairDft<16>::run(x);
+        else pair_factored<R1>(wt, x);
     }
     // inter-pass factors from the tile's table
     __device__ __forceinline__ static void twiddle(const float4 *tab, int t, int c, Pair (&x)[E]) {
@@ -196,7 +195,7 @@ struct PairTile : WarpTile<LOGR, LOGTILE, 4> {
             }
     }
     // back into the tile in natural row order, for a TMA store
-    __device__ __forceinline__ static void stage(uint8_t *tile, int t, int c, const Pair (&x)[E]) {
+    __device__ __forceinline__ static void stage(uint8_t *tile, int t, int c, const Pair (&x)[E], int) {
         constexpr int LR = S::logr(1), LP = S::logp(1), NB = E >> LR;
         const uint32_t off0 = warp_tile_off<LOGR, B::BOXC>((uint32_t)t, (uint32_t)c >> 1);
         __syncwarp();  // every lane has read its exchanged samples
@@ -207,6 +206,144 @@ struct PairTile : WarpTile<LOGR, LOGTILE, 4> {
                 const Pair &v = x[b + q * NB];
                 *(float4 *)(tile + off0 + (T * b + (q << LP)) * B::ROWB) =
                     make_float4(v.re.x, v.im.x, v.re.y, v.im.y);
+            }
+    }
+};
+
+// Two columns a thread, 16 samples of each, columns of 2^10 or 2^11 points over
+// T = 64 or 128 threads (two or four warps): three sub-passes (16 x 16 x 4 or 8),
+// whose exchanges meet at a named barrier of the column pair's warps.  2^11 rows
+// of 4 columns (32 bytes a row) make N = 2^21 and 2^22 two-pass transforms.
+template <int LOGR, int LOGTILE>
+struct WideTile {
+    using S = SubCfg<LOGR, 4>;
+    static_assert(S::NSUB == 3 && S::LOGT >= 6 && S::LOGT <= 7, "64 or 128 threads a column pair");
+    static constexpr int LE = 4, E = 16, R = 1 << LOGR, T = S::T, W = T / 32;
+    static constexpr bool SOA = true;
+    static constexpr int COLS = 1 << (LOGTILE - LOGR), BOXC = COLS, ROWB = BOXC * 8;
+    static_assert(COLS == 4 || COLS == 8, "one box a row");
+    static constexpr int WARPS = COLS / 2 * W;
+    static constexpr int TW_BYTES = COLS * (E + T) * (int)sizeof(float2);
+    // doubled table of sub-pass 1, plain one of sub-pass 2
+    static constexpr int R2 = 1 << S::logr(2), SUB1 = S::tw_count(1);
+    static constexpr int SUB_BYTES = SUB1 * 16 + S::tw_count(2) * 8;
+    using Values = Pair[E];
+
+    __device__ __forceinline__ static void fill_sub(uint8_t *tab, const float2 *__restrict__ tw, int tid, int nt) {
+        for (int i = tid; i < SUB1; i += nt) {
+            const float2 w = ld_tw(tw + i);
+            ((float4 *)tab)[i] = make_float4(w.x, w.x, w.y, w.y);
+        }
+        for (int i = tid; i < S::tw_count(2); i += nt) ((float2 *)(tab + SUB1 * 16))[i] = ld_tw(tw + SUB1 + i);
+    }
+    GBFFT_HD static void place(int warp, int lane, int &t, int &c) {
+        t = (warp % W) * 32 + lane;
+        c = 2 * (warp / W);
+    }
+    // Barrier of the column pair's T threads: names 1 .. 4 for group 0, 5 .. 8 for
+    // group 1 whatever the radix, so that the groups' tiles, which may differ in
+    // radix, never meet at one name with different thread counts.
+    __device__ __forceinline__ static void pair_sync(int c, int group) {
+        static_assert(COLS / 2 <= 4, "four barrier names a group");
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group * 4 + (c >> 1)), "n"(T) : "memory");
+    }
+    // rows of the exchange after sub-pass 0, as warp_xrow<4>: change of the read
+    // offset of row t + T e
+    GBFFT_HD static uint32_t read_xor(int t, int e) {
+        return warp_xor<BOXC>((uint32_t)((t >> 4) + (T / 16) * e) & 7u);
+    }
+    template <class Pre, class Read>
+    __device__ __forceinline__ static void run(uint8_t *tile, int t, int c, const uint8_t *sub, Pair (&x)[E], int group,
+                                               Pre pre, Read read) {
+        auto sync = [&] { pair_sync(c, group); };
+        const uint32_t off0 = warp_tile_off<LOGR, BOXC>((uint32_t)t, (uint32_t)c >> 1);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float4 q = *(const float4 *)(tile + off0 + e * (T * ROWB));
+            x[e] = Pair{make_float2(q.x, q.z), make_float2(q.y, q.w)};
+        }
+        pre(x);
+        PairDft<E>::run(x);
+        sync();  // the pair's threads have read their samples: its storage is free
+        const uint32_t offw = warp_tile_off<LOGR, BOXC>(((uint32_t)t << 4) | ((uint32_t)t & 7u), (uint32_t)c >> 1);
+#pragma unroll
+        for (int q = 0; q < E; ++q)
+            *(float4 *)(tile + (offw ^ warp_xor<BOXC>(q & 7)) + (q & ~7) * ROWB) =
+                make_float4(x[q].re.x, x[q].re.y, x[q].im.x, x[q].im.y);
+        sync();
+        const uint32_t offr = off0 ^ read_xor(t, 0);
+        const float4 *tw1 = (const float4 *)sub + (t & 15);
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float4 q = *(const float4 *)(tile + (offr ^ read_xor(0, e)) + e * (T * ROWB));
+            x[e] = Pair{make_float2(q.x, q.y), make_float2(q.z, q.w)};
+            if (e > 0) {
+                const float4 w = tw1[(e - 1) * 16];
+                x[e] = pair_mul(x[e], Pair{make_float2(w.x, w.y), make_float2(w.z, w.w)});
+            }
+        }
+        PairDft<E>::run(x);
+        sync();
+        const uint32_t off1 = warp_tile_off<LOGR, BOXC>((uint32_t)(((t >> 4) << 8) + (t & 15)), (uint32_t)c >> 1);
+#pragma unroll
+        for (int q = 0; q < E; ++q)
+            *(float4 *)(tile + off1 + q * (16 * ROWB)) = make_float4(x[q].re.x, x[q].re.y, x[q].im.x, x[q].im.y);
+        sync();
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float4 q = *(const float4 *)(tile + off0 + e * (T * ROWB));
+            x[e] = Pair{make_float2(q.x, q.y), make_float2(q.z, q.w)};
+        }
+        read();
+        Pair wt[R2];
+        const float2 *tw2 = (const float2 *)(sub + SUB1 * 16) + t;
+#pragma unroll
+        for (int m = 1; m < R2; ++m) {
+            const float2 w = tw2[(m - 1) * T];
+            wt[m] = Pair{pset(w.x), pset(w.y)};
+        }
+        pair_factored<R2>(wt, x);
+    }
+    __device__ __forceinline__ static void twiddle(const float4 *tab, int t, int c, Pair (&x)[E]) {
+        const float4 *f = tab + (c >> 1) * E;
+        const float4 wq = tab[COLS / 2 * E + ((c >> 1) << S::LOGT) + t];
+        const Pair w{make_float2(wq.x, wq.y), make_float2(wq.z, wq.w)};
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const float4 q = f[e];
+            x[e] = pair_mul(x[e], pair_mul(w, Pair{make_float2(q.x, q.y), make_float2(q.z, q.w)}));
+        }
+    }
+    __device__ __forceinline__ static void conj(Pair (&x)[E], float s) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) x[e].im = pmul(x[e].im, pset(s));
+    }
+    __device__ __forceinline__ static void scale(Pair (&x)[E], float re, float im) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) x[e] = Pair{pmul(x[e].re, pset(re)), pmul(x[e].im, pset(im))};
+    }
+    __device__ __forceinline__ static void store_columns(float2 *dst, int t, const Pair (&x)[E], uint64_t policy) {
+#pragma unroll
+        for (int b = 0; b < E / R2; ++b)
+#pragma unroll
+            for (int q = 0; q < R2; ++q) {
+                const Pair &v = x[b + q * (E / R2)];
+                float2 *d = dst + t + T * b + (q << 8);
+                st_policy(d, make_float2(v.re.x, v.im.x), policy);
+                st_policy(d + R, make_float2(v.re.y, v.im.y), policy);
+            }
+    }
+    // The pair's storage is read by other warps until all have passed sub-pass 2's
+    // reads: one more barrier before the results go back into it.
+    __device__ __forceinline__ static void stage(uint8_t *tile, int t, int c, const Pair (&x)[E], int group) {
+        pair_sync(c, group);
+        const uint32_t off0 = warp_tile_off<LOGR, BOXC>((uint32_t)t, (uint32_t)c >> 1);
+#pragma unroll
+        for (int b = 0; b < E / R2; ++b)
+#pragma unroll
+            for (int q = 0; q < R2; ++q) {
+                const Pair &v = x[b + q * (E / R2)];
+                *(float4 *)(tile + off0 + (T * b + (q << 8)) * ROWB) = make_float4(v.re.x, v.im.x, v.re.y, v.im.y);
             }
     }
 };
@@ -246,7 +383,7 @@ struct ColTile : WarpTile<LOGR, LOGTILE, 5> {
     }
     template <class Pre, class Read>
     __device__ __forceinline__ static void run(uint8_t *tile, int t, int c, const uint8_t *sub, float2 (&v)[E],
-                                               Pre pre, Read read) {
+                                               int, Pre pre, Read read) {
         DftRegs eng;
         const uint32_t off0 = off((uint32_t)t, (uint32_t)c);
 #pragma unroll
@@ -288,7 +425,7 @@ struct ColTile : WarpTile<LOGR, LOGTILE, 5> {
 #pragma unroll
             for (int q = 0; q < (1 << LR); ++q) st_policy(dst + t + T * b + (q << LP), v[b + q * NB], policy);
     }
-    __device__ __forceinline__ static void stage(uint8_t *tile, int t, int c, const float2 (&v)[E]) {
+    __device__ __forceinline__ static void stage(uint8_t *tile, int t, int c, const float2 (&v)[E], int) {
         constexpr int LR = S::logr(1), LP = S::logp(1), NB = E >> LR;
         const uint32_t off0 = off((uint32_t)t, (uint32_t)c);
         __syncwarp();

@@ -41,6 +41,7 @@ void DeviceBuffer::release() {
 Plan::~Plan() {
     if (tw) cudaFree(tw);
     if (fact) cudaFree(fact);
+    if (wide_fact) cudaFree(wide_fact);
     if (gtab) cudaFree(gtab);
 }
 
@@ -114,7 +115,12 @@ std::vector<PlanVariant> plan_candidates(int logn, int precision) {
     const bool tc = precision != GBFFT_PREC_FP32;
     const int top = tc ? 9 : 10;
     FusedDesc fd;
-    // three passes (L - 16, 8, 8) with the last two fused: the default where it exists
+    // 2^21 and 2^22 as two passes of radix 2^11 and 2^10 / 2^11 (fft_warp.cuh,
+    // WideTile): the first pass's HBM round trip goes (2^21 x 32: 464 -> 329 us,
+    // 2^22 x 16: 411 -> 346; 2^21 x 1: 30.7 -> 26.5).  2^23 would need tiles of 2^12
+    // rows, 16-byte rows in the same shared memory.
+    if (!tc && pipe_wide_info(logn, fd)) c.push_back(PlanVariant{11, false, true});
+    // three passes (L - 16, 8, 8) with the last two fused: the default elsewhere
     if (!tc && fused3_kernel_info(logn, fd)) {
         // its first pass with 32 samples a thread where that exists (radix 2^9 /
         // 2^10: N = 2^25, 2^26), measured faster (2^26: 114.9 vs 112.9 GSa/s)
@@ -140,7 +146,7 @@ std::vector<PlanVariant> plan_candidates(int logn, int precision) {
     for (int m = top; m >= 7; --m) {
         std::vector<int> parts = split_passes(logn, m);
         bool dup = false;
-        for (const PlanVariant &v : c) dup |= split_passes(logn, v.max_logr) == parts;
+        for (const PlanVariant &v : c) dup |= v.max_logr <= 10 && split_passes(logn, v.max_logr) == parts;
         if (dup || parts[0] < 5) continue;
         if (!tc) pass_order(parts);
         // the pair with 32 samples a thread (radix-32 sub-passes) first where a
@@ -211,7 +217,7 @@ int plan_build(Plan &p, int logn, int precision, const PlanVariant &v, cudaStrea
         p.multipass = true;
         p.needs_workspace = true;
         // the split form's radix-2^10 tile would not fit in shared memory
-        std::vector<int> parts = split_passes(logn, tc ? std::min(9, v.max_logr) : v.max_logr);
+        std::vector<int> parts = split_passes(logn, std::min(tc ? 9 : 10, v.max_logr));
         if (small_fused) parts = {7, logn - 7};
         if (!tc) pass_order(parts);
         const bool fused3 = v.fused && !tc && fused3_kernel_info(logn, p.fused);
@@ -266,6 +272,22 @@ int plan_build(Plan &p, int logn, int precision, const PlanVariant &v, cudaStrea
             }
             p.has_fused = p.fused.ctas_per_sm > 0;
         }
+        if (v.max_logr == 11 && p.has_fused && pipe_wide_info(logn, p.wide)) {
+            if ((e = fused_prepare(p.wide)) != cudaSuccess) {
+                why = cudaGetErrorString(e);
+                return GBFFT_ERR_CUDA;
+            }
+            for (int r : {p.wide.logra, p.wide.logrb}) {
+                TwiddleSegment ts[kMaxSub];
+                int entries = 0;
+                const int ns = pass_sub_segments(r, 4, ts, p.tw_entries, entries);
+                (r == p.wide.logra ? p.wide.sub_off_a : p.wide.sub_off_b) = (int64_t)p.tw_entries;
+                segs.insert(segs.end(), ts, ts + ns);
+                p.tw_entries += (uint64_t)entries;
+            }
+            if (p.wide.logra == p.wide.logrb) p.wide.sub_off_b = p.wide.sub_off_a;
+            p.has_wide = p.wide.pipe.ctas_per_sm > 0;
+        }
         if (tc) {
             if ((e = cudaMalloc(&p.gtab, kTcGtabBytes)) != cudaSuccess) {
                 cudaGetLastError();
@@ -287,6 +309,22 @@ int plan_build(Plan &p, int logn, int precision, const PlanVariant &v, cudaStrea
         if ((e = twiddle_fill(p.tw, segs.data(), (int)segs.size(), stream)) != cudaSuccess) {
             why = cudaGetErrorString(e);
             return GBFFT_ERR_CUDA;
+        }
+    }
+    if (p.has_wide) {
+        PipeDesc &wd = p.wide.pipe;
+        const uint64_t n = factors_count(p.wide.logrb, p.wide.logra, wd.loge);
+        if (cudaMalloc(&p.wide_fact, n * sizeof(float4)) != cudaSuccess) {
+            cudaGetLastError();  // no room: the three-pass form needs no factor table
+            p.wide_fact = nullptr;
+            p.has_wide = false;
+        } else {
+            if ((e = factors_fill(p.wide_fact, p.tw + p.tw_lo_offset, p.tw + p.tw_hi_offset, p.tw_split, logn,
+                                  p.wide.logrb, p.wide.logra, wd.loge, wd.logtile, wd.soa, stream)) != cudaSuccess) {
+                why = cudaGetErrorString(e);
+                return GBFFT_ERR_CUDA;
+            }
+            wd.fact_b = p.wide_fact;
         }
     }
     PipeDesc &pd = p.fused.pipe;
@@ -363,10 +401,12 @@ int plan_execute(const Plan &p, const float2 *in, float2 *out, uint64_t batch, i
     // Fused pass pair: both passes of a two-pass transform (out of place
     // only: its first pass writes into `out` while other tiles still read
     // `in`), or the last two of three after the first pass into the workspace.
-    const bool pair3 = p.has_fused && p.passes.size() == 3;
+    const bool wide = p.has_wide && ctr && wide_usable(in, out, ops) && batch <= 0x7fffffffull;
+    const FusedDesc &fd = wide ? p.wide : p.fused;
+    const bool pair3 = p.has_fused && p.passes.size() == 3 && !wide;
     const bool pair2 = p.has_fused && p.passes.size() == 2 && (const void *)in != (const void *)out;
-    const uint64_t ngroups = batch * p.fused.groups_per_transform;
-    if ((pair2 || pair3) && ctr && ngroups <= 0x7fffffffull) {
+    const uint64_t ngroups = batch * fd.groups_per_transform;
+    if ((pair2 || pair3 || wide) && ctr && ngroups <= 0x7fffffffull) {
         const size_t want = (2 + (size_t)ngroups) * sizeof(uint32_t);
         if (ctr->bytes < want) {
             int st = ctr->ensure(want, why);
@@ -395,10 +435,10 @@ int plan_execute(const Plan &p, const float2 *in, float2 *out, uint64_t batch, i
             ++launches;
             pair_in = (const float2 *)ws.ptr;
         }
-        const float2 *tw_a = p.fused.sub_off_a >= 0 ? p.tw + p.fused.sub_off_a : p.tw + p.passes[a].sub_tw_offset;
+        const float2 *tw_a = fd.sub_off_a >= 0 ? p.tw + fd.sub_off_a : p.tw + p.passes[a].sub_tw_offset;
         const float2 *tw_b =
-            p.fused.sub_off_b >= 0 ? p.tw + p.fused.sub_off_b : p.tw + p.passes[a + 1].sub_tw_offset;
-        e = fused_launch(p.fused, pair_in, out, batch, tw_a, tw_b, p.tw + p.tw_lo_offset, p.tw + p.tw_hi_offset,
+            fd.sub_off_b >= 0 ? p.tw + fd.sub_off_b : p.tw + p.passes[a + 1].sub_tw_offset;
+        e = fused_launch(fd, pair_in, out, batch, tw_a, tw_b, p.tw + p.tw_lo_offset, p.tw + p.tw_hi_offset,
                          (inv && !pair3) ? -1.0f : 1.0f, scale, inv ? -scale : 1.0f,
                          pair3 ? LoadOps{nullptr, 0u, 0.f, 0u} : ops, (uint32_t *)ctr->ptr, err, p.sms, stream,
                          p.gtab);

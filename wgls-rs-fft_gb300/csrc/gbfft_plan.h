@@ -82,7 +82,8 @@ struct FusedDesc {
 // Upper bound on the intermediates in flight between the two passes (bytes).
 constexpr uint64_t kFusedWindowBytes = 48ull << 20;
 
-// The tunable choices of a plan: largest global-pass radix (multi-pass split),
+// The tunable choices of a plan: largest global-pass radix (multi-pass split; 11: 2^21
+// and 2^22 as two passes),
 // whether kernels run as persistent tile loops with L2 prefetch, whether pass
 // pairs run as one launch with an L2-resident intermediate, and (single pass)
 // how many transforms a CTA takes.
@@ -120,10 +121,15 @@ struct Plan {
     std::vector<PassDesc> passes;
     bool has_fused = false;  // variant.fused and a kernel exists for the split
     FusedDesc fused;
+    // N = 2^21, 2^22 (max_logr 11): the transform as one two-pass launch, taken out of
+    // place on 16-byte boundaries without load options; the passes above otherwise
+    bool has_wide = false;
+    FusedDesc wide;
     // twiddle table (device): rows sub-pass tables, or for multi-pass the
     // per-pass sub-pass tables followed by the two-level W_N table.
     float2 *tw = nullptr;
     float4 *fact = nullptr;  // inter-pass factors of a warp-column pass pair
+    float4 *wide_fact = nullptr;
     uint64_t tw_entries = 0;
     uint64_t tw_lo_offset = 0, tw_hi_offset = 0;  // W_N^i (i < 2^s), W_N^{i 2^s}
     int tw_split = 0;                             // s
@@ -180,6 +186,10 @@ cudaError_t factors_fill(float4 *out, const float2 *lo, const float2 *hi, int sp
                          int loge, int logtile, bool soa, cudaStream_t stream);
 bool pipe2_kernel_info(int logr1, int logr2, PipeDesc &d, int loge);
 bool pipe3_kernel_info(int logn, PipeDesc &d);
+// N = 2^21, 2^22 as two passes of radix 2^11 and 2^(logn - 11)
+bool pipe_wide_info(int logn, FusedDesc &d);
+// Whether buffers and options suit that launch.
+bool wide_usable(const float2 *in, const float2 *out, const LoadOps &ops);
 // inflight: tiles that the launch's CTAs hold at once
 uint32_t fused_lag(uint64_t inflight, uint32_t tiles_per_group, uint64_t group_samples, uint64_t ngroups);
 cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint64_t batch, const float2 *tw_a,
