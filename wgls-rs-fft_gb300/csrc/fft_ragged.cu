@@ -26,6 +26,10 @@
 // a workspace.  Producers publish with a CTA barrier, then one thread's
 // __threadfence + atomicAdd; the consumer polls with ld.acquire.gpu and reads
 // the intermediate with L1-bypassing loads.
+//
+// Large FP32 sets of mostly two-pass transforms run out of place, on 16-byte
+// boundaries, as the warp-column form of the same queue (fft_ragged_pipe.cu;
+// rag_pipe_pays below has the rule).
 #include <algorithm>
 #include <cstring>
 #include <string>
@@ -33,60 +37,11 @@
 
 #include "gbfft_internal.h"
 #include "gbfft_plan.h"
-#include "gbfft_ragged.h"
+#include "fft_ragged.cuh"
 #include "fft_tc.cuh"
-#include "fft_tiles.cuh"
+#include "tensor_map.h"
 
 namespace gbfft {
-
-constexpr int kRagThreads = 512;
-constexpr int kRagMaxLogN = 18;
-constexpr int kRagRowsMaxLogN = 13;
-
-struct RagXform {
-    uint64_t offset;     // complex samples from the start of in/out
-    uint64_t ws_offset;  // two-pass transforms: start of their workspace slice
-    int32_t logn;
-    int32_t dir;         // GBFFT_FORWARD / GBFFT_INVERSE
-    uint32_t tiles1;     // two-pass transforms: number of first-pass items
-    uint32_t pad;
-};
-
-struct RagItem {
-    uint32_t kind;
-    uint32_t a;  // kind 0: first index into order[]; kind 1/2: transform id
-    uint32_t b;  // kind 0: transforms in the item;   kind 1/2: tile index
-    uint32_t logn;
-};
-
-struct RagParams {
-    const float2 *in;
-    float2 *out;
-    float2 *ws;
-    int p1_to_out;  // out of place: first-pass output goes to `out` (ws unused)
-    const RagItem *items;
-    uint32_t nitems;
-    uint32_t spin_limit;
-    const RagXform *xf;
-    const uint32_t *order;
-    uint32_t *item_counter;
-    uint32_t *done1;
-    uint32_t *error;
-    const float2 *sub[16];   // sub-pass tables of a length-2^L in-SMEM FFT
-    const float2 *lo[kRagMaxLogN + 1];
-    const float2 *hi[kRagMaxLogN + 1];
-    int split[kRagMaxLogN + 1];
-};
-
-__host__ __device__ constexpr int rag_logr1(int L) { return L / 2 + (L & 1); }
-__host__ __device__ constexpr int rag_logr2(int L) { return L / 2; }
-__host__ __device__ constexpr int rag_groups(int logr) { return kRagThreads / (kCols << (logr - 4)); }
-
-__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 
 template <int L>
 __device__ __forceinline__ void rag_rows(const RagParams &P, const RagItem &it, float2 *smem) {
@@ -317,7 +272,7 @@ struct RaggedPlanImpl {
     uint32_t spin_limit = 1u << 22;
     bool drop_producers = false;
     uint32_t lag_per_sm = 4;  // GBFFT_RAGGED_OPT_LAG
-    bool dirty = true;        // items must be (re)uploaded
+    bool dirty[2] = {true, true};  // [barrier, warp-column form]: its queue must be (re)uploaded
     std::vector<RagXform> xf;
     std::vector<RagItem> items;
     std::vector<uint32_t> order;
@@ -331,7 +286,7 @@ struct RaggedPlanImpl {
     DeviceBuffer tw;
     DeviceBuffer ws;
     uint32_t *h_error = nullptr;  // pinned copy of the error flag
-    size_t off_items = 0, off_order = 0, off_counters = 0, counters_bytes = 0;
+    size_t off_xf = 0, off_order = 0, off_counters = 0, counters_bytes = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     const void *g_in = nullptr;
@@ -342,6 +297,16 @@ struct RaggedPlanImpl {
     bool prepared = false;  // kernel attributes set
     int precision = GBFFT_PREC_FP32;
     void *gtab = nullptr;   // split form: the G operand parts (fft_passes_tc.cu)
+    // Warp-column form (fft_ragged_pipe.cu), taken out of place on 16-byte
+    // boundaries: FP32 plans with two-pass transforms, all of them at even offsets
+    bool pipe = false;
+    bool lag_set = false;     // GBFFT_RAGGED_OPT_LAG was given
+    uint64_t sub9_off = 0, sub13_off = 0;  // its 32-sample tables (need_sub9 / need_sub13)
+    bool need_sub9 = false, need_sub13 = false;
+    uint64_t fact_off[5] = {}, fact_entries = 0;  // inter-pass factors of 2^14 .. 2^18
+    DeviceBuffer fact;
+    std::vector<RagItem> pipe_items;  // the queue at this form's lag
+    size_t off_pitems = 0;
 };
 
 static int rag_tc_kind(const RaggedPlanImpl &p) { return tc_kind_of_precision(p.precision); }
@@ -371,8 +336,56 @@ static size_t rag_kernel_smem(const RaggedPlanImpl &p) {
     return p.precision == GBFFT_PREC_FP32 ? rag_smem_bytes() : rag_tc_smem_bytes(p);
 }
 
+// Default lag of the warp-column form, in items an SM.  Its loader runs two items
+// ahead of the groups and waits for a first pass without giving the slot up, so it
+// wants more distance than the barrier form: 1250 transforms of 2^8 .. 2^18 take 371
+// us at 3, 344 at 4, 320 at 6, 309 at 8, 317 at 10.
+constexpr uint32_t kRagPipeLag = 8;
+
+// When the warp-column form is the faster one (barrier form -> this form).  Two-pass
+// tiles gain once they fill the machine's slots a few times; until then the ring's
+// start-up is not paid back.  Groups of single-pass transforms lose: they are read
+// without the ring, by half as many threads.  In tiles an SM, two-pass + single-pass:
+//   2^16:        1.7 + 0  27.5 -> 25.7 us   3.4 + 0   36.2 -> 36.6    6.7 + 0  61 -> 51
+//   2^8..2^18:   3.4 + .1 38.1 -> 41.9      8.2 + .2  73.9 -> 71.8    47 + 1.5 370 -> 308
+//   2^8..2^17:   8.0 + .5 74.1 -> 75.0      16 + 1    138 -> 135      32 + 2   234 -> 221
+//   2^8..2^15:   10 + 3.3 98 -> 110
+static bool rag_pipe_pays(const RaggedPlanImpl &p) {
+    const uint64_t tile = 8192, rows = p.total_samples - p.ws_samples;
+    return p.ws_samples >= 6 * tile * (uint64_t)std::max(1, p.sms) + 8 * rows;
+}
+
+static void queue_items(const RaggedPlanImpl &p, const std::vector<RagItem> &rows, const std::vector<uint32_t> &two,
+                        uint64_t total_p1, uint32_t lag_per_sm, std::vector<RagItem> &items) {
+    items.clear();
+    // the second pass of a transform follows its first pass by `lag` items
+    const uint64_t lag = (uint64_t)lag_per_sm * (uint64_t)std::max(1, p.sms);
+    std::vector<std::pair<uint32_t, uint64_t>> pending;  // (transform, release position), FIFO
+    size_t head = 0, ri = 0;
+    uint64_t p1_seen = 0;
+    auto emit_p2 = [&](uint32_t i) {
+        const RagXform &x = p.xf[i];
+        const int lr2 = rag_logr2(x.logn);
+        const uint32_t tiles2 = (1u << (x.logn - lr2)) / (uint32_t)(kCols * rag_groups(lr2));
+        for (uint32_t t = 0; t < tiles2; ++t) items.push_back(RagItem{2, i, t, (uint32_t)x.logn});
+    };
+    for (uint32_t i : two) {
+        while (head < pending.size() && pending[head].second <= items.size()) emit_p2(pending[head++].first);
+        const RagXform &x = p.xf[i];
+        // test hook: nothing will publish the first pass
+        if (!p.drop_producers)
+            for (uint32_t t = 0; t < x.tiles1; ++t) items.push_back(RagItem{1, i, t, (uint32_t)x.logn});
+        p1_seen += x.tiles1;
+        pending.emplace_back(i, (uint64_t)items.size() + lag);
+        // single-pass groups in proportion to the first passes issued so far
+        const size_t want = (size_t)((double)rows.size() * (double)p1_seen / (double)total_p1);
+        while (ri < want && ri < rows.size()) items.push_back(rows[ri++]);
+    }
+    while (ri < rows.size()) items.push_back(rows[ri++]);
+    while (head < pending.size()) emit_p2(pending[head++].first);
+}
+
 static void build_items(RaggedPlanImpl &p) {
-    p.items.clear();
     p.order.clear();
     // kind 0: groups of whole transforms of one size, largest sizes first
     std::vector<std::vector<uint32_t>> by_size(kRagRowsMaxLogN + 1);
@@ -395,34 +408,11 @@ static void build_items(RaggedPlanImpl &p) {
     }
     uint64_t total_p1 = 0;
     for (uint32_t i : two) total_p1 += p.xf[i].tiles1;
-    // the second pass of a transform follows its first pass by `lag` items
-    const uint64_t lag = (uint64_t)p.lag_per_sm * (uint64_t)std::max(1, p.sms);
-    std::vector<std::pair<uint32_t, uint64_t>> pending;  // (transform, release position), FIFO
-    size_t head = 0, ri = 0;
-    uint64_t p1_seen = 0;
-    auto emit_p2 = [&](uint32_t i) {
-        const RagXform &x = p.xf[i];
-        const int lr2 = rag_logr2(x.logn);
-        const uint32_t tiles2 = (1u << (x.logn - lr2)) / (uint32_t)(kCols * rag_groups(lr2));
-        for (uint32_t t = 0; t < tiles2; ++t) p.items.push_back(RagItem{2, i, t, (uint32_t)x.logn});
-    };
-    for (uint32_t i : two) {
-        while (head < pending.size() && pending[head].second <= p.items.size()) emit_p2(pending[head++].first);
-        const RagXform &x = p.xf[i];
-        // test hook: nothing will publish the first pass
-        if (!p.drop_producers)
-            for (uint32_t t = 0; t < x.tiles1; ++t) p.items.push_back(RagItem{1, i, t, (uint32_t)x.logn});
-        p1_seen += x.tiles1;
-        pending.emplace_back(i, (uint64_t)p.items.size() + lag);
-        // single-pass groups in proportion to the first passes issued so far
-        const size_t want = (size_t)((double)rows.size() * (double)p1_seen / (double)total_p1);
-        while (ri < want && ri < rows.size()) p.items.push_back(rows[ri++]);
-    }
-    while (ri < rows.size()) p.items.push_back(rows[ri++]);
-    while (head < pending.size()) emit_p2(pending[head++].first);
+    queue_items(p, rows, two, total_p1, p.lag_per_sm, p.items);
+    if (p.pipe) queue_items(p, rows, two, total_p1, p.lag_set ? p.lag_per_sm : kRagPipeLag, p.pipe_items);
     if (p.order.empty()) p.order.push_back(0);
     p.nitems = (uint32_t)p.items.size();
-    p.dirty = true;
+    p.dirty[0] = p.dirty[1] = true;
 }
 
 int ragged_plan_build(RaggedPlanImpl *&out, int device, const gbfft_ragged_desc *descs, uint32_t count,
@@ -469,6 +459,9 @@ int ragged_plan_build(RaggedPlanImpl *&out, int device, const gbfft_ragged_desc 
         }
     }
     p->ws_samples = ws;
+    p->pipe = precision == GBFFT_PREC_FP32 && ws > 0 && rag_pipe_pays(*p);
+    for (const RagXform &x : p->xf)
+        if (x.logn > kRagRowsMaxLogN && (x.offset & 1u)) p->pipe = false;
     // twiddle tables
     uint64_t off = 0;
     for (int L = 0; L < 16; ++L) {
@@ -491,13 +484,38 @@ int ragged_plan_build(RaggedPlanImpl *&out, int device, const gbfft_ragged_desc 
         p->segs.push_back(TwiddleSegment{off, 1ull << (L - s), 1, L, 0, s});
         off += 1ull << (L - s);
     }
+    if (p->pipe) {
+        TwiddleSegment tmp[kMaxSub];
+        int entries = 0;
+        p->need_sub9 = p->need_2l[17] || p->need_2l[18];
+        p->need_sub13 = p->need_sub[13];
+        if (p->need_sub9) {
+            const int ns = pass_sub_segments(9, 5, tmp, off, entries);
+            p->segs.insert(p->segs.end(), tmp, tmp + ns);
+            p->sub9_off = off;
+            off += (uint64_t)entries;
+        }
+        if (p->need_sub13) {
+            const int ns = subcfg_segments<13, 5>(tmp, off);
+            p->segs.insert(p->segs.end(), tmp, tmp + ns);
+            p->sub13_off = off;
+            off += (uint64_t)SubCfg<13, 5>::tw_entries();
+        }
+        for (int L = 14; L <= kRagMaxLogN; ++L) {
+            if (!p->need_2l[L]) continue;
+            p->fact_off[L - 14] = p->fact_entries;
+            p->fact_entries += factors_count(rag_pipe_logr2(L), rag_pipe_logr1(L), rag_pipe_logr2(L) == 9 ? 5 : 4);
+        }
+    }
     p->tw_entries = off;
     build_items(*p);
     out = p;
     return GBFFT_OK;
 }
 
-int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, cudaStream_t stream, std::string &why) {
+// Makes the tables and copies the queue that a launch of this form takes.  `pipe` is
+// cleared where the warp-column form's tables find no room.
+static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cudaStream_t stream, std::string &why) {
     if (!p.prepared) {
         cudaError_t e = cudaFuncSetAttribute(rag_kernel(p), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)rag_kernel_smem(p));
@@ -531,31 +549,56 @@ int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, cudaStream_t stream, st
             }
         }
     }
+    if (pipe && !p.fact.ptr) {
+        std::string no_room;
+        cudaError_t e = ragged_pipe_prepare();
+        if (p.fact.ensure(p.fact_entries * sizeof(float4), no_room) != GBFFT_OK) {
+            p.pipe = pipe = false;  // the barrier form needs no factor table
+        } else {
+            const float2 *tw = (const float2 *)p.tw.ptr;
+            for (int L = 14; L <= kRagMaxLogN && e == cudaSuccess; ++L) {
+                if (!p.need_2l[L]) continue;
+                const bool col = rag_pipe_logr2(L) == 9;
+                e = factors_fill((float4 *)p.fact.ptr + p.fact_off[L - 14], tw + p.lo_off[L], tw + p.hi_off[L],
+                                 p.split[L], L, rag_pipe_logr2(L), rag_pipe_logr1(L), col ? 5 : 4, 13, !col, stream);
+            }
+        }
+        if (e != cudaSuccess) {
+            why = cudaGetErrorString(e);
+            return GBFFT_ERR_CUDA;
+        }
+    }
     if (in_place && p.ws_samples > 0) {  // out of place, the first pass writes into the output
         int st = p.ws.ensure(p.ws_samples * sizeof(float2), why);
         if (st != GBFFT_OK) return st;
     }
-    if (!p.dirty) return GBFFT_OK;
+    // [barrier form's queue | transforms | order | warp-column form's queue | counters]:
+    // each form takes the part that it needs in one copy, at its first launch
+    if (!p.dirty[pipe]) return GBFFT_OK;
     const size_t xf_bytes = p.xf.size() * sizeof(RagXform);
     const size_t it_bytes = p.items.size() * sizeof(RagItem);
     const size_t or_bytes = p.order.size() * sizeof(uint32_t);
-    p.off_items = (xf_bytes + 255) & ~(size_t)255;
-    p.off_order = (p.off_items + it_bytes + 255) & ~(size_t)255;
-    p.off_counters = (p.off_order + or_bytes + 255) & ~(size_t)255;
+    const size_t pi_bytes = p.pipe_items.size() * sizeof(RagItem);
+    p.off_xf = (it_bytes + 255) & ~(size_t)255;
+    p.off_order = (p.off_xf + xf_bytes + 255) & ~(size_t)255;
+    p.off_pitems = (p.off_order + or_bytes + 255) & ~(size_t)255;
+    p.off_counters = (p.off_pitems + pi_bytes + 255) & ~(size_t)255;
     p.counters_bytes = (2 + (size_t)p.count) * sizeof(uint32_t);
     int st = p.meta.ensure(p.off_counters + p.counters_bytes, why);
     if (st != GBFFT_OK) return st;
-    std::vector<char> host(p.off_counters, 0);
-    if (xf_bytes) memcpy(host.data(), p.xf.data(), xf_bytes);
-    if (it_bytes) memcpy(host.data() + p.off_items, p.items.data(), it_bytes);
-    memcpy(host.data() + p.off_order, p.order.data(), or_bytes);
-    cudaError_t e = cudaMemcpyAsync(p.meta.ptr, host.data(), host.size(), cudaMemcpyHostToDevice, stream);
+    const size_t from = pipe ? p.off_xf : 0, to = pipe ? p.off_counters : p.off_pitems;
+    std::vector<char> host(to - from, 0);
+    if (xf_bytes) memcpy(host.data() + (p.off_xf - from), p.xf.data(), xf_bytes);
+    memcpy(host.data() + (p.off_order - from), p.order.data(), or_bytes);
+    if (!pipe && it_bytes) memcpy(host.data(), p.items.data(), it_bytes);
+    if (pipe) memcpy(host.data() + (p.off_pitems - from), p.pipe_items.data(), pi_bytes);
+    cudaError_t e = cudaMemcpyAsync((char *)p.meta.ptr + from, host.data(), host.size(), cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) {
         why = cudaGetErrorString(e);
         return GBFFT_ERR_CUDA;
     }
-    p.dirty = false;
+    p.dirty[pipe] = false;
     return GBFFT_OK;
 }
 
@@ -567,10 +610,10 @@ static RagParams rag_params(const RaggedPlanImpl &p, const void *in, void *out) 
     P.out = (float2 *)out;
     P.ws = (float2 *)p.ws.ptr;
     P.p1_to_out = in != (const void *)out;
-    P.items = (const RagItem *)(m + p.off_items);
+    P.items = (const RagItem *)m;
     P.nitems = p.nitems;
     P.spin_limit = p.spin_limit;
-    P.xf = (const RagXform *)m;
+    P.xf = (const RagXform *)(m + p.off_xf);
     P.order = (const uint32_t *)(m + p.off_order);
     uint32_t *ctr = (uint32_t *)(m + p.off_counters);
     P.item_counter = ctr;
@@ -587,12 +630,23 @@ static RagParams rag_params(const RaggedPlanImpl &p, const void *in, void *out) 
 }
 
 // Enqueue counters reset + persistent launch + error-flag readback on `s`.
-static cudaError_t rag_enqueue(RaggedPlanImpl &p, const void *in, void *out, cudaStream_t s) {
+static cudaError_t rag_enqueue(RaggedPlanImpl &p, const void *in, void *out, bool pipe, cudaStream_t s) {
     char *m = (char *)p.meta.ptr;
     cudaError_t e = cudaMemsetAsync(m + p.off_counters, 0, p.counters_bytes, s);
     if (e != cudaSuccess) return e;
     RagParams P = rag_params(p, in, out);
-    if (p.nitems > 0) {
+    if (p.nitems > 0 && pipe) {
+        RagPipeTables t;
+        memset(&t, 0, sizeof t);
+        const float2 *tw = (const float2 *)p.tw.ptr;
+        t.sub9 = p.need_sub9 ? tw + p.sub9_off : nullptr;
+        t.sub13 = p.need_sub13 ? tw + p.sub13_off : nullptr;
+        for (int L = 14; L <= kRagMaxLogN; ++L)
+            if (p.need_2l[L]) t.fact[L - 14] = (const float4 *)p.fact.ptr + p.fact_off[L - 14];
+        P.items = (const RagItem *)(m + p.off_pitems);
+        e = ragged_pipe_launch(P, t, p.max_extent, p.sms, s);
+        if (e != cudaSuccess) return e;
+    } else if (p.nitems > 0) {
         // two resident CTAs per SM, one for the TF32 split form (its A operands
         // take twice the shared memory)
         const int per_sm = p.precision == GBFFT_PREC_TC_TF32 ? 1 : 2;
@@ -609,11 +663,12 @@ static cudaError_t rag_enqueue(RaggedPlanImpl &p, const void *in, void *out, cud
 
 int ragged_plan_execute(RaggedPlanImpl &p, const void *in, void *out, cudaStream_t stream, bool use_graph,
                         std::string &why) {
-    int st = ragged_plan_upload(p, in == (const void *)out, stream, why);
+    bool pipe = p.pipe && in != (const void *)out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && tensor_map_encoder();
+    int st = ragged_plan_upload(p, in == (const void *)out, pipe, stream, why);
     if (st != GBFFT_OK) return st;
     cudaError_t e;
     if (!use_graph) {
-        e = rag_enqueue(p, in, out, stream);
+        e = rag_enqueue(p, in, out, pipe, stream);
         if (e != cudaSuccess) {
             why = cudaGetErrorString(e);
             return GBFFT_ERR_CUDA;
@@ -635,7 +690,7 @@ int ragged_plan_execute(RaggedPlanImpl &p, const void *in, void *out, cudaStream
         }
         e = cudaStreamBeginCapture(p.capture_stream, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            cudaError_t e2 = rag_enqueue(p, in, out, p.capture_stream);
+            cudaError_t e2 = rag_enqueue(p, in, out, pipe, p.capture_stream);
             e = cudaStreamEndCapture(p.capture_stream, &p.graph);
             if (e2 != cudaSuccess) e = e2;
         }
@@ -689,6 +744,7 @@ int ragged_plan_set(RaggedPlanImpl &p, int option, uint64_t value, std::string &
                 return GBFFT_ERR_INVALID_ARGUMENT;
             }
             p.lag_per_sm = (uint32_t)value;
+            p.lag_set = true;
             build_items(p);
             break;
         default:

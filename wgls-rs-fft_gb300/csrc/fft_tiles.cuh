@@ -12,6 +12,21 @@
 
 namespace gbfft {
 
+// Threads of a rows tile: the whole CTA, or (an engine with `group_threads`) a
+// group of that many consecutive threads with its own barrier.
+template <class Eng>
+__device__ __forceinline__ void tile_sync(Eng &eng) {
+    if constexpr (requires { eng.group_threads; })
+        asm volatile("bar.sync %0, %1;" ::"r"(eng.barrier), "n"(Eng::group_threads) : "memory");
+    else
+        __syncthreads();
+}
+template <class Eng>
+__device__ __forceinline__ int tile_thread(Eng &eng) {
+    if constexpr (requires { eng.group_threads; }) return (int)threadIdx.x % Eng::group_threads;
+    else return (int)threadIdx.x;
+}
+
 constexpr int kColsLog = 4;
 constexpr int kCols = 1 << kColsLog;
 
@@ -31,13 +46,13 @@ struct RowsChain {
     template <class Eng>
     __device__ __forceinline__ static void run(float2 (&v)[C::E], int t, float2 *buf, const float2 *tw, Eng &eng) {
         constexpr int PR = C::logr(I - 1), PP = C::logp(I - 1);  // previous sub-pass
-        if (I > 1) __syncthreads();  // readers of the previous exchange are done
+        if (I > 1) tile_sync(eng);  // readers of the previous exchange are done
 #pragma unroll
         for (int b = 0; b < (C::E >> PR); ++b)
 #pragma unroll
             for (int q = 0; q < (1 << PR); ++q)
                 buf[swz<C::LOGE>(subpass_out_pos<PR, PP, C::LOGT>(t, b, q), PP)] = v[b + q * (C::E >> PR)];
-        __syncthreads();
+        tile_sync(eng);
 #pragma unroll
         for (int e = 0; e < C::E; ++e) v[e] = buf[swz<C::LOGE>(t + C::T * e, PP)];
         subpass_run<LOGN, I, LE>(v, t, tw, eng);
@@ -83,7 +98,7 @@ template <int LOGN, int G, int DIRC = 0, int LE = 4, class RefFn, class Eng = Df
 __device__ __forceinline__ void rows_tile(RefFn ref, const float2 *__restrict__ tw, float2 *smem, const LoadOps &ops,
                                           Eng eng = Eng()) {
     using C = SubCfg<LOGN, LE>;
-    const int tid = threadIdx.x;
+    const int tid = tile_thread(eng);
     const int g = tid >> C::LOGT;
     const int t = tid & (C::T - 1);
     const RowRef r = ref(g);
