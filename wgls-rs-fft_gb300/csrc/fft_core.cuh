@@ -275,4 +275,19 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
+// Every kernel that launch_overlapped starts begins with one of these (after set-up that
+// reads a plan's tables only); neither has an effect in an ordinary launch.
+// stream_wait: wait for the launches before it in the stream.  The next launch is
+// brought up as this one's CTAs leave.
+// stream_order: that, and let the next launch be brought up at once -- in this order, so
+// that whatever is brought up has only this launch left to wait for.  For the
+// single-pass kernels (split form, 2^8 x 64 FP16: 4.64 us against 4.79, 2^13 x 8 TF32 12.5
+// against 12.8); the pairs run their last tiles beside CTAs that wait, and lose (2^24 x 4:
+// 473 us against 428, 2^16 x 1024 FP16 480 against 477).
+__device__ __forceinline__ void stream_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void stream_order() {
+    stream_wait();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 }  // namespace gbfft

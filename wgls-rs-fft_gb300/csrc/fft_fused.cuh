@@ -230,6 +230,7 @@ __device__ __forceinline__ void fused_finish(const FusedParams &P, int *flag) {
 template <int LOGRA, int LOGRB, int THREADS, int LOGN, int LOGPA, int LE = 4>
 __global__ void __launch_bounds__(THREADS, (FusedCfg<LOGRA, LOGRB, THREADS, LOGN, LOGPA, LE>::MINB))
 fft_fused_kernel(FusedParams P) {
+    stream_wait();
     extern __shared__ float2 smem_f[];
     // packed FP32 butterflies (2^16: 226 -> 232 GSa/s), except for pairs with a
     // radix-2^10 pass (32 x 32 sub-passes at 128 registers), where the scalar

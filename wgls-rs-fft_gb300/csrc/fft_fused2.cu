@@ -148,8 +148,8 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
     P.gtab = (const uint4 *)gtab;
     // The warp-column form (fft_pipe.cuh) needs tensor maps: buffers on 16-byte
     // boundaries, and no tables of row addresses.  It is the faster one wherever
-    // its ring of tiles fills (2^16 x 1024: 297 -> 237 us, 2^16 x 32: 21.6 ->
-    // 21.2), but takes longer to start: a launch of no more tiles than resident
+    // its ring of tiles fills (2^16 x 1024: 297 -> 230 us, 2^16 x 32: 21.6 ->
+    // 17.1), but takes longer to start: a launch of no more tiles than resident
     // CTAs, or of a single group (no second pass can start before the whole first
     // one is done), is left to the barrier form (2^16 x 4: 12.3 against 10.3 us,
     // 2^20 x 1: 21.5 against 20.5).  Load options stay with the barrier form, whose
@@ -171,7 +171,7 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
             Q.fact_b = d.pipe.fact_b;
             Q.f = P;
             void *args[] = {(void *)&Q};
-            return cudaLaunchKernel(d.pipe.fn, dim3((unsigned)std::min<uint64_t>(P.nitems, pipe_ctas)),
+            return launch_overlapped(d.pipe.fn, dim3((unsigned)std::min<uint64_t>(P.nitems, pipe_ctas)),
                                     dim3(d.pipe.threads), args, d.pipe.smem, stream);
         }
     }
@@ -181,7 +181,7 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
     P.lag = fused_lag(ctas, d.tiles_per_group, d.group_samples, P.ngroups);
     const uint64_t grid = std::min<uint64_t>((uint64_t)P.nitems, ctas);
     void *args[] = {(void *)&P};
-    return cudaLaunchKernel(d.fn, dim3((unsigned)grid), dim3(d.threads), args, d.smem, stream);
+    return launch_overlapped(d.fn, dim3((unsigned)grid), dim3(d.threads), args, d.smem, stream);
 }
 
 }  // namespace gbfft

@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(PassCfg<LOGR, LE, CL>::THREADS, PassCfg<LOGR, 
 fft_pass_kernel(const float2 *in, float2 *out, int logn, int logp, const float2 *__restrict__ tw,
                 const float2 *__restrict__ tw_lo, const float2 *__restrict__ tw_hi, int tw_split,
                 float in_im_sign, float out_re_scale, float out_im_scale, LoadOps ops) {
+    stream_wait();
     extern __shared__ __align__(16) float2 smem_pass[];
     const int lognc = logn - LOGR;                     // log2 (columns per transform)
     const uint64_t tile = blockIdx.x;
@@ -80,6 +81,7 @@ fft_pass_persistent_kernel(const float2 *in, float2 *out, int logn, int logp, co
                            const float2 *__restrict__ tw_lo, const float2 *__restrict__ tw_hi, int tw_split,
                            float in_im_sign, float out_re_scale, float out_im_scale, LoadOps ops,
                            uint64_t ntiles) {
+    stream_wait();
     extern __shared__ __align__(16) float2 smem_pass[];
     constexpr int R = 1 << LOGR;
     const int lognc = logn - LOGR;
@@ -149,6 +151,7 @@ fft_pass_first_tma_kernel(const __grid_constant__ CUtensorMap map, float2 *out, 
                           const float2 *__restrict__ tw, const float2 *__restrict__ tw_lo,
                           const float2 *__restrict__ tw_hi, int tw_split, float in_im_sign, LoadOps ops,
                           uint32_t *err) {
+    stream_wait();
     using T = PassTmaCfg<LOGR, LE>;
     constexpr int R = 1 << LOGR;
     extern __shared__ __align__(1024) float2 smem_tma[];
@@ -222,6 +225,7 @@ fft_pass_first_tma_persistent_kernel(const __grid_constant__ CUtensorMap map, fl
                                      const float2 *__restrict__ tw, const float2 *__restrict__ tw_lo,
                                      const float2 *__restrict__ tw_hi, int tw_split, float in_im_sign, LoadOps ops,
                                      uint32_t *err, uint64_t ntiles) {
+    stream_wait();
     using T = PassTmaCfg<LOGR, LE>;
     constexpr int R = 1 << LOGR;
     extern __shared__ __align__(1024) float2 smem_tma[];
@@ -430,12 +434,12 @@ cudaError_t pass_launch(const PassDesc &d, const float2 *in, float2 *out, uint64
                 void *pargs[] = {(void *)&map,   (void *)&out,      (void *)&logn,       (void *)&tw_sub,
                                  (void *)&tw_lo, (void *)&tw_hi,    (void *)&tw_split,   (void *)&in_im_sign,
                                  (void *)&ops,   (void *)&err,      (void *)&tiles};
-                return cudaLaunchKernel(d.fn_tma_persistent, dim3((unsigned)grid), dim3(d.threads), pargs,
+                return launch_overlapped(d.fn_tma_persistent, dim3((unsigned)grid), dim3(d.threads), pargs,
                                         d.smem_tma, stream);
             }
             void *args[] = {(void *)&map,  (void *)&out,   (void *)&logn,     (void *)&tw_sub,     (void *)&tw_lo,
                             (void *)&tw_hi, (void *)&tw_split, (void *)&in_im_sign, (void *)&ops, (void *)&err};
-            return cudaLaunchKernel(d.fn_tma, dim3((unsigned)tiles), dim3(d.threads), args, d.smem_tma, stream);
+            return launch_overlapped(d.fn_tma, dim3((unsigned)tiles), dim3(d.threads), args, d.smem_tma, stream);
         }
     }
     if (persistent && d.fn_persistent && d.persist_ctas_per_sm > 0 && sms > 0) {
@@ -444,13 +448,13 @@ cudaError_t pass_launch(const PassDesc &d, const float2 *in, float2 *out, uint64
                         (void *)&tw_sub, (void *)&tw_lo, (void *)&tw_hi,   (void *)&tw_split,
                         (void *)&in_im_sign, (void *)&out_re_scale, (void *)&out_im_scale, (void *)&ops,
                         (void *)&tiles};
-        return cudaLaunchKernel(d.fn_persistent, dim3((unsigned)grid), dim3(d.threads), args, d.smem, stream);
+        return launch_overlapped(d.fn_persistent, dim3((unsigned)grid), dim3(d.threads), args, d.smem, stream);
     }
     if (tiles > 0x7fffffffull) return cudaErrorInvalidConfiguration;
     void *args[] = {(void *)&in,    (void *)&out,   (void *)&logn,     (void *)&logp,
                     (void *)&tw_sub, (void *)&tw_lo, (void *)&tw_hi,   (void *)&tw_split,
                     (void *)&in_im_sign, (void *)&out_re_scale, (void *)&out_im_scale, (void *)&ops};
-    return cudaLaunchKernel(d.fn, dim3((unsigned)tiles), dim3(d.threads), args, d.smem, stream);
+    return launch_overlapped(d.fn, dim3((unsigned)tiles), dim3(d.threads), args, d.smem, stream);
 }
 
 }  // namespace gbfft

@@ -124,6 +124,7 @@ fft_pass_tc_kernel(const float2 *in, float2 *out, int logn, int logp, const floa
                    const float2 *__restrict__ tw_lo, const float2 *__restrict__ tw_hi, int tw_split,
                    float in_im_sign, float out_re_scale, float out_im_scale, const uint4 *__restrict__ gtab,
                    uint32_t *err, LoadOps ops) {
+    stream_wait();
     using C = PassTcCfg<LOGR, KIND>;
     extern __shared__ __align__(1024) uint8_t smem_tc[];
     TcState st;
@@ -170,6 +171,7 @@ struct FusedTcCfg {
 template <int LOGRA, int LOGRB, int THREADS, int LOGN, int KIND, int LE = 4>
 __global__ void __launch_bounds__(THREADS, (FusedTcCfg<LOGRA, LOGRB, THREADS, LOGN, KIND, LE>::MINB))
 fft_fused_tc_kernel(FusedParams P) {
+    stream_wait();
     using C = FusedTcCfg<LOGRA, LOGRB, THREADS, LOGN, KIND, LE>;
     extern __shared__ __align__(1024) uint8_t smem_ftc[];
     TcState st;
@@ -233,7 +235,7 @@ cudaError_t pass_tc_launch(const PassDesc &d, const float2 *in, float2 *out, uin
                     (void *)&tw_sub, (void *)&tw_lo, (void *)&tw_hi,     (void *)&tw_split,
                     (void *)&in_im_sign, (void *)&out_re_scale, (void *)&out_im_scale, (void *)&gtab,
                     (void *)&err, (void *)&ops};
-    return cudaLaunchKernel(d.fn, dim3((unsigned)tiles), dim3(d.threads), args, d.smem, stream);
+    return launch_overlapped(d.fn, dim3((unsigned)tiles), dim3(d.threads), args, d.smem, stream);
 }
 
 template <int LOGRA, int LOGRB, int THREADS, int KIND, int LE = 4>

@@ -381,6 +381,7 @@ fft_pipe_kernel(const __grid_constant__ PipeParams P) {
     }
     C::KA::fill_sub(smem_pipe + C::OFF_SUBA, P.f.tw_a, threadIdx.x, C::THREADS);
     if (C::OFF_SUBB != C::OFF_SUBA) C::KB::fill_sub(smem_pipe + C::OFF_SUBB, P.f.tw_b, threadIdx.x, C::THREADS);
+    stream_wait();  // (the tables above are complete before a plan's first launch)
     __syncthreads();
     if (warp == C::COMPUTE) {
         if (lane == 0) pipe_loader<C, LOGPA>(P, smem_pipe, B);

@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(RowsCfg<LOGN, LOGS, LE>::THREADS, RowsCfg<LOGN
 fft_rows_persistent_kernel(const float2 *in, float2 *out, uint64_t batch, const float2 *__restrict__ tw,
                            float in_im_sign, float out_re_scale, float out_im_scale, LoadOps ops,
                            const uint64_t *, const uint64_t *) {  // (no row tables: the host never passes them)
+    stream_order();
     using C = RowsCfg<LOGN, LOGS, LE>;
     extern __shared__ float2 smem_rows[];
     constexpr uint32_t kTileSamples = C::G * C::N;
@@ -147,7 +148,7 @@ cudaError_t rows_launch(const RowsKernelInfo &k, const float2 *in, float2 *out, 
     float out_re = scale, out_im = inv ? -scale : 1.0f;
     void *args[] = {(void *)&in,     (void *)&out,    (void *)&batch, (void *)&tw,     (void *)&in_im,
                     (void *)&out_re, (void *)&out_im, (void *)&ops,   (void *)&tab_in, (void *)&tab_out};
-    return cudaLaunchKernel(fn, dim3((unsigned)ctas), dim3(k.threads), args, k.smem, stream);
+    return launch_overlapped(fn, dim3((unsigned)ctas), dim3(k.threads), args, k.smem, stream);
 }
 
 }  // namespace gbfft

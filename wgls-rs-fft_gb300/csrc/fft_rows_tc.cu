@@ -48,10 +48,10 @@ cudaError_t rows_tc_launch(const RowsKernelInfo &k, const float2 *in, float2 *ou
     const uint64_t resident = (uint64_t)k.persist_ctas_per_sm * (uint64_t)std::max(1, sms);
     const uint64_t tiles = (batch + k.persist_transforms - 1) / k.persist_transforms;
     if (k.fn_persistent && tiles >= 3 * resident)
-        return cudaLaunchKernel(inv ? k.fn_persistent_inv : k.fn_persistent, dim3((unsigned)resident),
+        return launch_overlapped(inv ? k.fn_persistent_inv : k.fn_persistent, dim3((unsigned)resident),
                                 dim3(k.persist_threads), args, k.persist_smem, stream);
     const uint64_t ctas = (batch + k.transforms_per_cta - 1) / k.transforms_per_cta;
-    return cudaLaunchKernel(inv ? k.fn_inv : k.fn, dim3((unsigned)ctas), dim3(k.threads), args, k.smem, stream);
+    return launch_overlapped(inv ? k.fn_inv : k.fn, dim3((unsigned)ctas), dim3(k.threads), args, k.smem, stream);
 }
 
 }  // namespace gbfft

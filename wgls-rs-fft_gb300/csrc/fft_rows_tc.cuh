@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(RowsTcCfg<LOGN, KIND, LOOP>::THREADS, RowsTcCf
 fft_rows_tc_kernel(const float2 *in, float2 *out, uint64_t batch, const float2 *__restrict__ tw,
                    float in_im_sign, float out_re_scale, float out_im_scale, LoadOps ops,
                    const uint4 *__restrict__ gtab, uint32_t *err) {
+    stream_order();
     using C = RowsTcCfg<LOGN, KIND, LOOP>;
     using Gm = TcGeom<KIND>;
     extern __shared__ __align__(1024) uint8_t smem_rtc[];

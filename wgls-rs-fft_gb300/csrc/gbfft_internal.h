@@ -52,6 +52,10 @@ struct RowsKernelInfo {
     int nseg = 0;
     int tw_entries = 0;
 };
+// A kernel that begins with stream_order(), brought up while the launch before it in
+// the stream still runs; it touches no memory before that one is complete (twiddle.cu).
+cudaError_t launch_overlapped(const void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t stream);
+
 // logs: log2 of the samples a CTA moves (12; 11 or 13 for N = 2^6 .. 2^11);
 // loge: log2 of the samples a thread holds (4; 5 for N = 2^13, 2^14)
 bool rows_kernel_info(int logn, RowsKernelInfo &k, int logs = 12, int loge = 4);
