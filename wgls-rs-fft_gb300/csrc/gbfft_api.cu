@@ -17,6 +17,7 @@
 #include <map>
 #include <mutex>
 #include <memory>
+#include <optional>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -101,6 +102,7 @@ struct gbfft_ctx {
     // plans by (logn, precision, variant); tuned variant by (logn, precision, direction, log2 batch)
     std::map<std::tuple<int, int, PlanVariant>, std::unique_ptr<Plan>> plans;
     std::map<std::tuple<int, int, int, int>, PlanVariant> tuned;
+    std::map<std::pair<int, int>, std::optional<PlanVariant>> untuned;  // (log2 N, precision): first candidate
     int window = GBFFT_WINDOW_NONE;
     uint32_t noise_seed = 0;
     float noise_sigma = 0.f;  // 0: no noise added on load
@@ -272,7 +274,9 @@ PlanVariant choose_variant(gbfft_ctx *ctx, int logn, uint64_t batch, int directi
         it = ctx->tuned.find(tune_key(ctx, logn, batch, direction));
         if (st == GBFFT_OK && it != ctx->tuned.end()) return it->second;
     }
-    return plan_candidates(logn, ctx->precision).front();
+    std::optional<PlanVariant> &v = ctx->untuned[{logn, ctx->precision}];
+    if (!v) v = plan_candidates(logn, ctx->precision).front();
+    return *v;
 }
 
 // The window table for 2^logn samples when a window is selected, else nullptr.

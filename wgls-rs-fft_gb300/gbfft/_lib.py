@@ -1,17 +1,20 @@
 """ctypes binding of the C ABI in include/gbfft.h.
 
-There is no fallback: if libgbfft.so is missing or cannot be loaded, every
+Context.c2c_device, the call whose own cost shows, goes through a small extension module
+(``_call.c``) where that is built.  There is no fallback for the library: if libgbfft.so is missing or cannot be loaded, every
 entry point raises.  The library is the only implementation of the transform.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import threading
 
 import numpy as np
 
-from .build import LIB_PATH
+from .build import CALL_PATH, LIB_PATH
 
 FORWARD = -1
 INVERSE = +1
@@ -65,6 +68,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_c2c = None  # _call.c's c2c, where it is built
 _lock = threading.Lock()
 
 
@@ -82,7 +86,7 @@ def lib_path() -> str:
 
 def load():
     """Load libgbfft.so (raises if it is absent -- there is no CPU path)."""
-    global _lib
+    global _lib, _c2c
     with _lock:
         if _lib is None:
             path = lib_path()
@@ -93,6 +97,12 @@ def load():
                 f = getattr(L, name)
                 f.restype = res
                 f.argtypes = args
+            if os.path.exists(CALL_PATH):
+                loader = importlib.machinery.ExtensionFileLoader("_gbfft_call", CALL_PATH)
+                spec = importlib.util.spec_from_loader("_gbfft_call", loader)
+                module = importlib.util.module_from_spec(spec)
+                loader.exec_module(module)
+                _c2c = module.c2c
             _lib = L
         return _lib
 
@@ -123,9 +133,13 @@ class Context:
         if st != OK:
             raise GbfftError(st, status_string(st))
         self._h = h
+        self._c2c = _c2c
+        self._c2c_fn = ctypes.cast(self._L.gbfft_c2c_device, _vp).value
+        self._c2c_ctx = h.value
 
     def close(self):
         if getattr(self, "_h", None):
+            self._c2c = None
             self._L.gbfft_destroy(self._h)
             self._h = None
 
@@ -195,6 +209,12 @@ class Context:
     def c2c_device(self, d_in, d_out, n: int, batch: int, direction: int = FORWARD, stream=None):
         """Enqueue on device pointers (ints or tensors).  `stream` is a
         cudaStream_t as an int; None or 0 is the CUDA default stream."""
+        if self._c2c is not None:
+            st = self._c2c(self._c2c_fn, self._c2c_ctx, d_in, d_out, n, batch, direction, stream)
+            if st == OK:
+                return
+            if st is not None:
+                self._check(st)
         s = 0 if stream is None else int(stream)
         self._check(self._L.gbfft_c2c_device(self._h, _ptr(d_in), _ptr(d_out), n, batch, direction, s or None))
 

@@ -9,6 +9,7 @@ import concurrent.futures as cf
 import os
 import shutil
 import subprocess
+import sysconfig
 
 PKG_ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 REPO_ROOT = os.path.dirname(PKG_ROOT)
@@ -16,6 +17,8 @@ CSRC = os.path.join(PKG_ROOT, "csrc")
 LIB_DIR = os.path.join(PKG_ROOT, "lib")
 OBJ_DIR = os.path.join(PKG_ROOT, "_build")
 LIB_PATH = os.path.join(LIB_DIR, "libgbfft.so")
+CALL_SRC = os.path.join(PKG_ROOT, "gbfft", "_call.c")
+CALL_PATH = os.path.join(LIB_DIR, "_gbfft_call.so")
 INCLUDE = os.path.join(REPO_ROOT, "include")
 
 ARCH_FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -60,6 +63,21 @@ def _compile(src: str, verbose: bool) -> str:
     return obj
 
 
+def _build_call(force: bool) -> None:
+    """The interpreter-side call (``_call.c``); without Python's headers or a C compiler
+    the binding makes its calls through ctypes."""
+    include = sysconfig.get_paths()["include"]
+    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
+    if not cc or not os.path.exists(os.path.join(include, "Python.h")):
+        return
+    if not force and os.path.exists(CALL_PATH) and os.path.getmtime(CALL_PATH) >= os.path.getmtime(CALL_SRC):
+        return
+    r = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-Wall", "-I", include, "-o", CALL_PATH, CALL_SRC],
+                       capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{cc} failed on _call.c:\n{r.stdout}\n{r.stderr}")
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile (if stale) and link libgbfft.so; returns its path."""
     os.makedirs(OBJ_DIR, exist_ok=True)
@@ -77,6 +95,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _build_call(force)
     return LIB_PATH
 
 
