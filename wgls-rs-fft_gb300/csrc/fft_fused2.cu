@@ -2,6 +2,7 @@
 // (N = 2^15 .. 2^20, both passes in one launch) and the host side shared with
 // the three-pass pairs (fft_fused3.cu).
 #include <algorithm>
+#include <cstring>
 
 #include "gbfft_internal.h"
 #include "gbfft_plan.h"
@@ -121,6 +122,44 @@ static bool pipe_map(CUtensorMap *map, const void *base, uint64_t cols, uint64_t
                   // us; 32, 128 and 256 bytes 359, 359, 363)
                   box_cols >= 8 ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B : CU_TENSOR_MAP_L2_PROMOTION_L2_64B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The first pass alone of a transform of 2^logn samples, through the ring of tiles of a
+// shorter pair whose pass A has its radix: the queue is cut off before the first B
+// item.  A group is as many columns as that pair's transform has: group g's tiles are
+// columns g N' / R .. of the long transform (the maps' third dimension), and its
+// output the next N' samples.  One transform a launch: two dimensions of the map are
+// its rows and the groups.  For N = 2^26, whose radix-2^10 first pass ran one CTA an SM
+// in lock-step (194 us where radix 2^9 takes 164): 2^26 x 1 470.6 -> 460 us.  Needs what
+// the wide pairs need (wide_usable); the pass kernel otherwise.
+cudaError_t pipe_first_launch(const FusedDesc &d, const float2 *in, float2 *out, int logn, const float2 *tw_a,
+                              float in_im, uint32_t *ctr, uint32_t *err, int sms, cudaStream_t stream) {
+    PipeParams Q;
+    memset(&Q, 0, sizeof Q);
+    const uint64_t cols = 1ull << (d.logn - d.logra);
+    PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
+    const cuuint64_t dims[3] = {2 * cols, 1ull << d.logra, 1ull << (logn - d.logn)};
+    const cuuint64_t strides[2] = {sizeof(float2) << (logn - d.logra), cols * sizeof(float2)};
+    const cuuint32_t box[3] = {(cuuint32_t)(2 * d.pipe.box_cols_a), 256, 1}, estr[3] = {1, 1, 1};
+    if (!encode || encode(&Q.map_in, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)in, dims, strides, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return cudaErrorInvalidValue;
+    FusedParams &P = Q.f;
+    P.in = in;
+    P.out = out;
+    P.batch = P.ngroups = P.lag = 1u << (logn - d.logn);
+    P.nitems = d.pipe.tiles_per_group * P.ngroups;
+    P.tw_a = P.tw_b = tw_a;
+    P.in_im = in_im;
+    P.out_re = P.out_im = 1.0f;
+    P.ctr = ctr;
+    P.err = err;
+    P.spin_limit = 1u << 22;
+    void *args[] = {(void *)&Q};
+    const uint64_t ctas = (uint64_t)d.pipe.ctas_per_sm * (uint64_t)std::max(1, sms);
+    return launch_overlapped(d.pipe.fn, dim3((unsigned)std::min<uint64_t>(P.nitems, ctas)), dim3(d.pipe.threads), args,
+                             d.pipe.smem, stream);
 }
 
 cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint64_t batch, const float2 *tw_a,

@@ -272,6 +272,16 @@ int plan_build(Plan &p, int logn, int precision, const PlanVariant &v, cudaStrea
             }
             p.has_fused = p.fused.ctas_per_sm > 0;
         }
+        if (p.has_fused && parts.size() == 3 && parts[0] == 10 && v.loge == 5 && v.tma && !v.persistent &&
+            pipe2_kernel_info(10, 10, p.lone.pipe, 5)) {
+            p.lone.logra = p.lone.logrb = 10;
+            p.lone.logn = 20;
+            if ((e = fused_prepare(p.lone)) != cudaSuccess) {
+                why = cudaGetErrorString(e);
+                return GBFFT_ERR_CUDA;
+            }
+            p.has_lone = p.lone.pipe.ctas_per_sm > 0;
+        }
         if (v.max_logr == 11 && p.has_fused && pipe_wide_info(logn, p.wide)) {
             if ((e = fused_prepare(p.wide)) != cudaSuccess) {
                 why = cudaGetErrorString(e);
@@ -425,9 +435,19 @@ int plan_execute(const Plan &p, const float2 *in, float2 *out, uint64_t batch, i
             int st = ws.ensure(((size_t)batch << p.logn) * sizeof(float2), why);
             if (st != GBFFT_OK) return st;
             const PassDesc &d0 = p.passes[0];
-            e = pass_launch(d0, in, (float2 *)ws.ptr, batch, p.logn, p.tw + d0.sub_tw_offset, p.tw + p.tw_lo_offset,
-                            p.tw + p.tw_hi_offset, p.tw_split, inv ? -1.0f : 1.0f, 1.0f, 1.0f, stream,
-                            p.variant.persistent, p.sms, ops, err);
+            // (its counters, one a 2^20 samples, are no more than the pair's: one a 2^20)
+            if (p.has_lone && wide_usable(in, (const float2 *)ws.ptr, ops)) {
+                e = cudaSuccess;
+                for (uint64_t b = 0; b < batch && e == cudaSuccess; ++b)
+                    e = pipe_first_launch(p.lone, in + (b << p.logn), (float2 *)ws.ptr + (b << p.logn), p.logn,
+                                          p.tw + d0.sub_tw_offset, inv ? -1.0f : 1.0f, (uint32_t *)ctr->ptr, err,
+                                          p.sms, stream);
+                launches += batch - 1;
+            } else {
+                e = pass_launch(d0, in, (float2 *)ws.ptr, batch, p.logn, p.tw + d0.sub_tw_offset,
+                                p.tw + p.tw_lo_offset, p.tw + p.tw_hi_offset, p.tw_split, inv ? -1.0f : 1.0f, 1.0f,
+                                1.0f, stream, p.variant.persistent, p.sms, ops, err);
+            }
             if (e != cudaSuccess) {
                 why = cudaGetErrorString(e);
                 return GBFFT_ERR_CUDA;

@@ -125,6 +125,10 @@ struct Plan {
     // place on 16-byte boundaries without load options; the passes above otherwise
     bool has_wide = false;
     FusedDesc wide;
+    // N = 2^26: its first pass (radix 2^10) through the ring of tiles, pass A of the
+    // 2^20 pair alone
+    bool has_lone = false;
+    FusedDesc lone;
     // twiddle table (device): rows sub-pass tables, or for multi-pass the
     // per-pass sub-pass tables followed by the two-level W_N table.
     float2 *tw = nullptr;
@@ -192,6 +196,8 @@ bool pipe_wide_info(int logn, FusedDesc &d);
 bool wide_usable(const float2 *in, const float2 *out, const LoadOps &ops);
 // inflight: tiles that the launch's CTAs hold at once
 uint32_t fused_lag(uint64_t inflight, uint32_t tiles_per_group, uint64_t group_samples, uint64_t ngroups);
+cudaError_t pipe_first_launch(const FusedDesc &d, const float2 *in, float2 *out, int logn, const float2 *tw_a,
+                              float in_im, uint32_t *ctr, uint32_t *err, int sms, cudaStream_t stream);
 cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint64_t batch, const float2 *tw_a,
                          const float2 *tw_b, const float2 *tw_lo, const float2 *tw_hi, float in_im, float out_re,
                          float out_im, LoadOps ops, uint32_t *ctr, uint32_t *err, int sms, cudaStream_t stream,
