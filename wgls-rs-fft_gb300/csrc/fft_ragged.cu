@@ -10,7 +10,7 @@
 //   kind 2  second global pass of such a transform, 16*NG columns
 // The queue mixes first passes and single-pass groups in proportion, and
 // places the second pass of each transform a fixed number of items after its
-// first pass (twice the CTAs in flight): late enough that it rarely waits,
+// first pass (four an SM): late enough that it rarely waits,
 // early enough that the first pass's output, stored with normal L2 priority,
 // is still in L2 when it is read back.  Every CTA claims items in queue order
 // with one atomicAdd (the next claim is made while the current item runs).
