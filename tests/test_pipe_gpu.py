@@ -15,7 +15,7 @@ TOL_REL_L2 = 2e-6
 
 
 @pytest.mark.parametrize("logn,batch", [(15, 20), (15, 301), (16, 11), (16, 203), (17, 5), (17, 67), (18, 3), (18, 33),
-                                        (19, 2), (19, 13), (20, 2), (20, 5), (21, 1), (21, 3), (22, 1), (22, 3), (23, 1),
+                                        (19, 1), (19, 2), (19, 13), (20, 2), (20, 5), (21, 1), (21, 3), (22, 1), (22, 3), (23, 1),
                                         (24, 1), (25, 1), (26, 1), (26, 2)])
 def test_pipe_matches_barrier_form_and_fp64(lib_built, logn, batch):
     import gbfft

@@ -187,15 +187,19 @@ cudaError_t fused_launch(const FusedDesc &d, const float2 *in, float2 *out, uint
     P.gtab = (const uint4 *)gtab;
     // The warp-column form (fft_pipe.cuh) needs tensor maps: buffers on 16-byte
     // boundaries, and no tables of row addresses.  It is the faster one wherever
-    // its ring of tiles fills (2^16 x 1024: 297 -> 230 us, 2^16 x 32: 21.6 ->
-    // 17.1), but takes longer to start: a launch of no more tiles than resident
-    // CTAs, or of a single group (no second pass can start before the whole first
-    // one is done), is left to the barrier form (2^16 x 4: 12.3 against 10.3 us,
-    // 2^20 x 1: 21.5 against 20.5).  Load options stay with the barrier form, whose
-    // lanes run along the columns: here they run along the rows, and each window
-    // factor would be a sector of its own (2^16 x 1024: 342 against 315 us).
+    // its ring of tiles fills (2^16 x 1024: 297 -> 230 us, 2^16 x 32: 21.0 -> 17.0),
+    // but takes longer to start: a launch of no more tiles than resident CTAs, or of
+    // a single group (no second pass can start before the whole first one is done),
+    // is left to the barrier form (2^16 x 4: 9.4 us here against 8.1, 2^17 x 4 12.7
+    // against 11.7, 2^20 x 1 18.5 against 18.2).  Except where every tile has a CTA of
+    // its own and the barrier form's are radix-2^10 tiles, whose 16 warps go through
+    // them in lock-step: 2^19 x 1 13.7 us here against 17.5.  Load options stay with
+    // the barrier form, whose lanes run along the columns: here they run along the
+    // rows, and each window factor would be a sector of its own (2^16 x 1024: 342
+    // against 315 us).
     const uint64_t pipe_ctas = (uint64_t)d.pipe.ctas_per_sm * (uint64_t)std::max(1, sms);
-    const bool filled = P.ngroups > 1 && 2ull * d.pipe.tiles_per_group * P.ngroups > pipe_ctas;
+    const uint64_t tiles = 2ull * d.pipe.tiles_per_group * P.ngroups;
+    const bool filled = tiles > pipe_ctas ? P.ngroups > 1 : d.logra == 10;
     if (d.pipe.fn && !tab_in && !tab_out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && (filled || !d.fn) &&
         !(d.pipe.first && (ops.win || ops.noise_sigma != 0.f))) {
         PipeParams Q;
