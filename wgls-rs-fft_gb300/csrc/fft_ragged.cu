@@ -171,8 +171,11 @@ __device__ __forceinline__ void rag_loop(const RagParams &P, float2 *smem_rag, E
 // (gtab and off_g are the tensor-core kernel's; both kernels take the same arguments)
 __global__ void __launch_bounds__(kRagThreads, 2) fft_ragged_kernel(RagParams P, const uint4 *, uint32_t) {
     extern __shared__ float2 smem_rag[];
+    stream_wait();
     DftRegs eng;
     rag_loop(P, smem_rag, eng);
+    __shared__ int s_last;
+    rag_finish<kRagThreads>(P, &s_last);
 }
 
 // Tensor-core split forms.  Shared memory: the item region (FP32 exchange
@@ -194,6 +197,7 @@ __global__ void __launch_bounds__(kRagThreads, (KIND == kTcTF32 ? 1 : 2))
 fft_ragged_tc_kernel(RagParams P, const uint4 *__restrict__ gtab, uint32_t off_g) {
     using Lay = RagTcLayout<KIND>;
     using Gm = TcGeom<KIND>;
+    stream_wait();
     extern __shared__ __align__(1024) uint8_t smem_rtc[];
     uint64_t *bar = (uint64_t *)(smem_rtc + off_g + Gm::PARTS * Gm::G_BYTES);
     uint32_t *s_taddr = (uint32_t *)(smem_rtc + off_g + Gm::PARTS * Gm::G_BYTES + 8);
@@ -232,6 +236,7 @@ fft_ragged_tc_kernel(RagParams P, const uint4 *__restrict__ gtab, uint32_t off_g
     __syncthreads();
     tc_fence_after();
     if (tid < 32) tmem_dealloc(st.taddr, Lay::TMEM_COLS);
+    rag_finish<kRagThreads>(P, s_abort);
 }
 
 // ---------------------------------------------------------------------------
@@ -583,7 +588,7 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
     p.off_order = (p.off_xf + xf_bytes + 255) & ~(size_t)255;
     p.off_pitems = (p.off_order + or_bytes + 255) & ~(size_t)255;
     p.off_counters = (p.off_pitems + pi_bytes + 255) & ~(size_t)255;
-    p.counters_bytes = (2 + (size_t)p.count) * sizeof(uint32_t);
+    p.counters_bytes = (3 + (size_t)p.count) * sizeof(uint32_t);
     int st = p.meta.ensure(p.off_counters + p.counters_bytes, why);
     if (st != GBFFT_OK) return st;
     const size_t from = pipe ? p.off_xf : 0, to = pipe ? p.off_counters : p.off_pitems;
@@ -593,6 +598,8 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
     if (!pipe && it_bytes) memcpy(host.data(), p.items.data(), it_bytes);
     if (pipe) memcpy(host.data() + (p.off_pitems - from), p.pipe_items.data(), pi_bytes);
     cudaError_t e = cudaMemcpyAsync((char *)p.meta.ptr + from, host.data(), host.size(), cudaMemcpyHostToDevice, stream);
+    // (from then on every launch leaves them zero)
+    if (e == cudaSuccess) e = cudaMemsetAsync((char *)p.meta.ptr + p.off_counters, 0, p.counters_bytes, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess) {
         why = cudaGetErrorString(e);
@@ -618,7 +625,10 @@ static RagParams rag_params(const RaggedPlanImpl &p, const void *in, void *out) 
     uint32_t *ctr = (uint32_t *)(m + p.off_counters);
     P.item_counter = ctr;
     P.error = ctr + 1;
-    P.done1 = ctr + 2;
+    P.exits = ctr + 2;
+    P.done1 = ctr + 3;
+    P.counters = 3 + p.count;
+    P.host_error = p.h_error;
     const float2 *tw = (const float2 *)p.tw.ptr;
     for (int L = 0; L < 16; ++L) P.sub[L] = p.need_sub[L] ? tw + p.sub_off[L] : nullptr;
     for (int L = 0; L <= kRagMaxLogN; ++L) {
@@ -629,13 +639,13 @@ static RagParams rag_params(const RaggedPlanImpl &p, const void *in, void *out) 
     return P;
 }
 
-// Enqueue counters reset + persistent launch + error-flag readback on `s`.
+// Enqueue the persistent launch on `s`.
 static cudaError_t rag_enqueue(RaggedPlanImpl &p, const void *in, void *out, bool pipe, cudaStream_t s) {
     char *m = (char *)p.meta.ptr;
-    cudaError_t e = cudaMemsetAsync(m + p.off_counters, 0, p.counters_bytes, s);
-    if (e != cudaSuccess) return e;
+    if (p.nitems == 0)  // nothing to launch: a node for the graph
+        return cudaMemsetAsync(m + p.off_counters, 0, p.counters_bytes, s);
     RagParams P = rag_params(p, in, out);
-    if (p.nitems > 0 && pipe) {
+    if (pipe) {
         RagPipeTables t;
         memset(&t, 0, sizeof t);
         const float2 *tw = (const float2 *)p.tw.ptr;
@@ -644,21 +654,16 @@ static cudaError_t rag_enqueue(RaggedPlanImpl &p, const void *in, void *out, boo
         for (int L = 14; L <= kRagMaxLogN; ++L)
             if (p.need_2l[L]) t.fact[L - 14] = (const float4 *)p.fact.ptr + p.fact_off[L - 14];
         P.items = (const RagItem *)(m + p.off_pitems);
-        e = ragged_pipe_launch(P, t, p.max_extent, p.sms, s);
-        if (e != cudaSuccess) return e;
-    } else if (p.nitems > 0) {
-        // two resident CTAs per SM, one for the TF32 split form (its A operands
-        // take twice the shared memory)
-        const int per_sm = p.precision == GBFFT_PREC_TC_TF32 ? 1 : 2;
-        const unsigned grid = (unsigned)std::max(1, std::min<int>(per_sm * p.sms, (int)p.nitems));
-        const uint4 *gtab = (const uint4 *)p.gtab;
-        uint32_t off_g = (uint32_t)rag_tc_off_g(p);
-        void *args[] = {(void *)&P, (void *)&gtab, (void *)&off_g};
-        e = cudaLaunchKernel(rag_kernel(p), dim3(grid), dim3(kRagThreads), args, rag_kernel_smem(p), s);
-        if (e != cudaSuccess) return e;
+        return ragged_pipe_launch(P, t, p.max_extent, p.sms, s);
     }
-    return cudaMemcpyAsync(p.h_error, m + p.off_counters + sizeof(uint32_t), sizeof(uint32_t),
-                           cudaMemcpyDeviceToHost, s);
+    // two resident CTAs per SM, one for the TF32 split form (its A operands
+    // take twice the shared memory)
+    const int per_sm = p.precision == GBFFT_PREC_TC_TF32 ? 1 : 2;
+    const unsigned grid = (unsigned)std::max(1, std::min<int>(per_sm * p.sms, (int)p.nitems));
+    const uint4 *gtab = (const uint4 *)p.gtab;
+    uint32_t off_g = (uint32_t)rag_tc_off_g(p);
+    void *args[] = {(void *)&P, (void *)&gtab, (void *)&off_g};
+    return launch_overlapped(rag_kernel(p), dim3(grid), dim3(kRagThreads), args, rag_kernel_smem(p), s);
 }
 
 int ragged_plan_execute(RaggedPlanImpl &p, const void *in, void *out, cudaStream_t stream, bool use_graph,

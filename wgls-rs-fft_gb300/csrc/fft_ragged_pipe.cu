@@ -16,8 +16,7 @@
 // What is left is the pass pairs' own bound (data written, read back and rewritten
 // through L2) and the two tile radices a size mix alternates between.  96 registers a
 // thread; the bodies of 2^9 .. 2^13 single-pass groups spill, which a mix with few of
-// them does not see.  Waiting, publication and bounded waits as in fft_pipe.cuh; the
-// counters are reset before every launch.
+// them does not see.  Waiting, publication and bounded waits as in fft_pipe.cuh.
 #include <algorithm>
 #include <cstring>
 
@@ -271,64 +270,65 @@ __global__ void __launch_bounds__(RagPipe::THREADS, 1) fft_ragged_pipe_kernel(co
     if (P.r.sub[7]) C::K7::fill_sub(smem_rp + C::OFF_SUB7, P.r.sub[7], threadIdx.x, C::THREADS);
     if (P.r.sub[8]) C::K8::fill_sub(smem_rp + C::OFF_SUB8, P.r.sub[8], threadIdx.x, C::THREADS);
     if (P.t.sub9) C::K9::fill_sub(smem_rp + C::OFF_SUB9, P.t.sub9, threadIdx.x, C::THREADS);
+    stream_wait();  // (the tables above are complete before a plan's first launch)
     __syncthreads();
     if (warp == C::COMPUTE) {
         if (lane == 0) rag_loader(P, smem_rp, B);
-        return;
-    }
-    if (warp == C::COMPUTE + 1) {
+    } else if (warp == C::COMPUTE + 1) {
         if (lane == 0) rag_storer(P, smem_rp, B);
-        return;
-    }
-    const int cg = warp / C::WPG, wg = warp % C::WPG;
-    RagGroup eng;
-    eng.barrier = 1 + cg;
-    for (uint32_t i = (uint32_t)cg;; i += C::GROUPS) {
-        const uint32_t s = i % S;
-        // the group's warps share a barrier: they go on or leave together
-        const bool ok = __all_sync(0xffffffffu, pipe_wait(B.full + i % D, (i / D) & 1u, B.abort));
-        if (!group_all(3 + cg, C::WPG * 32, ok)) {
-            if (lane == 0) {
-                *B.abort = 1;
-                atomicExch(P.r.error, 1u);
+    } else {
+        const int cg = warp / C::WPG, wg = warp % C::WPG;
+        RagGroup eng;
+        eng.barrier = 1 + cg;
+        for (uint32_t i = (uint32_t)cg;; i += C::GROUPS) {
+            const uint32_t s = i % S;
+            // the group's warps share a barrier: they go on or leave together
+            const bool ok = __all_sync(0xffffffffu, pipe_wait(B.full + i % D, (i / D) & 1u, B.abort));
+            if (!group_all(3 + cg, C::WPG * 32, ok)) {
+                if (lane == 0) {
+                    *B.abort = 1;
+                    atomicExch(P.r.error, 1u);
+                }
+                break;
             }
-            break;
-        }
-        const volatile RagPipeItem &it = B.item[i % D];
-        const uint32_t kind = it.kind;
-        uint8_t *slot = smem_rp + s * C::TILE_BYTES;
-        if (kind == 0) {
-            switch (it.logn) {
+            const volatile RagPipeItem &it = B.item[i % D];
+            const uint32_t kind = it.kind;
+            uint8_t *slot = smem_rp + s * C::TILE_BYTES;
+            if (kind == 0) {
+                switch (it.logn) {
 #define GBFFT_RP_ROWS(L) \
-    case L: rag_group_rows<L, 4>(P.r, P.r.sub[L], it, (float2 *)slot, eng); break;
-                GBFFT_RP_ROWS(0) GBFFT_RP_ROWS(1) GBFFT_RP_ROWS(2) GBFFT_RP_ROWS(3) GBFFT_RP_ROWS(4)
-                GBFFT_RP_ROWS(5) GBFFT_RP_ROWS(6) GBFFT_RP_ROWS(7) GBFFT_RP_ROWS(8) GBFFT_RP_ROWS(9)
-                GBFFT_RP_ROWS(10) GBFFT_RP_ROWS(11) GBFFT_RP_ROWS(12)
+        case L: rag_group_rows<L, 4>(P.r, P.r.sub[L], it, (float2 *)slot, eng); break;
+                    GBFFT_RP_ROWS(0) GBFFT_RP_ROWS(1) GBFFT_RP_ROWS(2) GBFFT_RP_ROWS(3) GBFFT_RP_ROWS(4)
+                    GBFFT_RP_ROWS(5) GBFFT_RP_ROWS(6) GBFFT_RP_ROWS(7) GBFFT_RP_ROWS(8) GBFFT_RP_ROWS(9)
+                    GBFFT_RP_ROWS(10) GBFFT_RP_ROWS(11) GBFFT_RP_ROWS(12)
 #undef GBFFT_RP_ROWS
-                case 13: rag_group_rows<13, 5>(P.r, P.t.sub13, it, (float2 *)slot, eng); break;
-                default: break;
+                    case 13: rag_group_rows<13, 5>(P.r, P.t.sub13, it, (float2 *)slot, eng); break;
+                    default: break;
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(B.free + s);
+            } else if (kind != kRagEnd) {
+                const int logr = kind == 1 ? rag_pipe_logr1(it.logn) : rag_pipe_logr2(it.logn);
+                const float4 *tab = (const float4 *)(smem_rp + C::OFF_TW + s * C::TW_BYTES);
+                if (logr == 7) {
+                    // (second passes of radix 2^7 are 2^14's: factors from global memory)
+                    rag_tile<C::K7, 7>(P, it, slot, smem_rp + C::OFF_SUB7,
+                                       P.t.fact[0] + (size_t)it.tile * (C::K7::TW_BYTES / 16), cg, wg, lane, B.free + s);
+                } else if (logr == 8) {
+                    rag_tile<C::K8, 8>(P, it, slot, smem_rp + C::OFF_SUB8, tab, cg, wg, lane, B.free + s);
+                } else {
+                    rag_tile<C::K9, 9>(P, it, slot, smem_rp + C::OFF_SUB9, tab, cg, wg, lane, B.free + s);
+                }
+                fence_proxy_async_smem();  // this lane's accesses of the slot before the TMA's
             }
-            fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0) mbar_arrive(B.free + s);
-        } else if (kind != kRagEnd) {
-            const int logr = kind == 1 ? rag_pipe_logr1(it.logn) : rag_pipe_logr2(it.logn);
-            const float4 *tab = (const float4 *)(smem_rp + C::OFF_TW + s * C::TW_BYTES);
-            if (logr == 7) {
-                // (second passes of radix 2^7 are 2^14's: factors from global memory)
-                rag_tile<C::K7, 7>(P, it, slot, smem_rp + C::OFF_SUB7,
-                                   P.t.fact[0] + (size_t)it.tile * (C::K7::TW_BYTES / 16), cg, wg, lane, B.free + s);
-            } else if (logr == 8) {
-                rag_tile<C::K8, 8>(P, it, slot, smem_rp + C::OFF_SUB8, tab, cg, wg, lane, B.free + s);
-            } else {
-                rag_tile<C::K9, 9>(P, it, slot, smem_rp + C::OFF_SUB9, tab, cg, wg, lane, B.free + s);
-            }
-            fence_proxy_async_smem();  // this lane's accesses of the slot before the TMA's
+            if (lane == 0) mbar_arrive(B.done + i % D);
+            if (kind == kRagEnd) break;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(B.done + i % D);
-        if (kind == kRagEnd) break;
     }
+    __syncthreads();  // (s_abort is no longer read)
+    rag_finish<C::THREADS>(P.r, s_abort);
 }
 
 }  // namespace
@@ -360,7 +360,7 @@ cudaError_t ragged_pipe_launch(const RagParams &P, const RagPipeTables &t, uint6
         }
     }
     void *args[] = {(void *)&Q};
-    return cudaLaunchKernel((const void *)fft_ragged_pipe_kernel, dim3(std::min<unsigned>(P.nitems, (unsigned)std::max(1, sms))),
+    return launch_overlapped((const void *)fft_ragged_pipe_kernel, dim3(std::min<unsigned>(P.nitems, (unsigned)std::max(1, sms))),
                          dim3(RagPipe::THREADS), args, RagPipe::SMEM, stream);
 }
 
