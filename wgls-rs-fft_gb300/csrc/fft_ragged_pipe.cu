@@ -327,6 +327,9 @@ __global__ void __launch_bounds__(RagPipe::THREADS, 1) fft_ragged_pipe_kernel(co
             if (kind == kRagEnd) break;
         }
     }
+    // the loader's and the storer's other lanes are here already: the barrier below is a
+    // whole warp's
+    __syncwarp();
     __syncthreads();  // (s_abort is no longer read)
     rag_finish<C::THREADS>(P.r, s_abort);
 }

@@ -16,10 +16,12 @@ namespace gbfft {
 // group of that many consecutive threads with its own barrier.
 template <class Eng>
 __device__ __forceinline__ void tile_sync(Eng &eng) {
-    if constexpr (requires { eng.group_threads; })
+    if constexpr (requires { eng.group_threads; }) {
+        __syncwarp();  // bar.sync is a whole warp's: lanes without a transform skip loads and stores
         asm volatile("bar.sync %0, %1;" ::"r"(eng.barrier), "n"(Eng::group_threads) : "memory");
-    else
+    } else {
         __syncthreads();
+    }
 }
 template <class Eng>
 __device__ __forceinline__ int tile_thread(Eng &eng) {
