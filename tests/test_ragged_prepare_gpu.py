@@ -1,0 +1,73 @@
+"""GPU: what a ragged plan keeps between calls is complete or not there."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL_REL_L2 = 2e-6
+
+
+def _descs(sizes, seed=5):
+    """Transforms of these log2 sizes back to back, directions mixed, at even offsets."""
+    rng = np.random.default_rng(seed)
+    descs, off = [], 2
+    for L in sizes:
+        descs.append((off, int(L), int(rng.choice([-1, 1]))))
+        off += max(2, 1 << int(L))
+    return descs, off
+
+
+def _large(seed=5):
+    """Enough two-pass transforms of 2^14 .. 2^18 for the ring (fft_ragged.cu, rag_pipe_pays)."""
+    rng = np.random.default_rng(seed)
+    return _descs(list(rng.permutation(list(range(8, 19)) + [int(v) for v in rng.choice(range(14, 19), 130)])), seed)
+
+
+def _small():
+    return _descs(list(range(19)))
+
+
+def _data(torch, total):
+    x = torch.view_as_complex(torch.randn(total, 2, generator=torch.Generator("cuda").manual_seed(total), device="cuda"))
+    return x, torch.full_like(x, float("nan"))
+
+
+def _check(torch, x, y, descs):
+    for off, L, d in descs:
+        a = x[off:off + (1 << L)].to(torch.complex128)
+        want = torch.fft.fft(a) if d < 0 else torch.fft.ifft(a)
+        err = (torch.linalg.vector_norm(y[off:off + (1 << L)] - want) / torch.linalg.vector_norm(want)).item()
+        assert err <= TOL_REL_L2, (off, L, d, err)
+
+
+@pytest.mark.parametrize("prec,large", [(0, False), (0, True), (1, False)])
+def test_tables_after_a_first_call_under_capture(lib_built, prec, large):
+    """A plan's first call makes its tables and cannot be captured; it is refused, and the
+    next ordinary call makes them."""
+    import gbfft
+    torch = pytest.importorskip("torch")
+    descs, total = _large() if large else _small()
+    x, y = _data(torch, total)
+    with gbfft.Context(0) as ctx:
+        ctx.set_precision(prec)
+        plan = ctx.ragged_plan(descs)
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="relaxed")
+            try:
+                with pytest.raises(gbfft.GbfftError):
+                    plan.execute(x, y, total, use_graph=False, stream=stream.cuda_stream)
+            finally:
+                try:
+                    graph.capture_end()
+                except RuntimeError:
+                    ctx._L.cudaGetLastError()
+        ctx._L.cudaGetLastError()
+        for graphed in (False, True):
+            y.fill_(float("nan"))
+            torch.cuda.synchronize()
+            plan.execute(x, y, total, use_graph=graphed)
+            plan.wait()
+            _check(torch, x, y, descs)
+        plan.close()

@@ -299,7 +299,9 @@ struct RaggedPlanImpl {
     cudaStream_t capture_stream = nullptr;
     uint64_t launches = 0;
     int sms = 0;
-    bool prepared = false;  // kernel attributes set
+    // Tables that a launch may read.  Set when the stream that filled them has been waited
+    // for: an allocated table may be a failed call's, or its fill may have gone into a capture.
+    bool filled = false, fact_filled = false;
     int precision = GBFFT_PREC_FP32;
     void *gtab = nullptr;   // split form: the G operand parts (fft_passes_tc.cu)
     // Warp-column form (fft_ragged_pipe.cu), taken out of place on 16-byte
@@ -518,21 +520,33 @@ int ragged_plan_build(RaggedPlanImpl *&out, int device, const gbfft_ragged_desc 
     return GBFFT_OK;
 }
 
+static bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return false;
+}
+
 // Makes the tables and copies the queue that a launch of this form takes.  `pipe` is
 // cleared where the warp-column form's tables find no room.
 static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cudaStream_t stream, std::string &why) {
-    if (!p.prepared) {
+    const bool fill = !p.filled;
+    bool fill_fact = pipe && !p.fact_filled;
+    if ((fill || fill_fact || p.dirty[pipe]) && capturing(stream)) {
+        why = "a ragged plan's first call fills its tables and cannot be captured";
+        return GBFFT_ERR_CUDA;
+    }
+    if (fill) {
         cudaError_t e = cudaFuncSetAttribute(rag_kernel(p), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)rag_kernel_smem(p));
         if (e == cudaSuccess && p.precision != GBFFT_PREC_FP32) {
-            e = cudaMalloc(&p.gtab, kTcGtabBytes);
+            if (!p.gtab) e = cudaMalloc(&p.gtab, kTcGtabBytes);
             if (e == cudaSuccess) e = tc_gtab_fill(p.gtab, stream);
         }
         if (e != cudaSuccess) {
             why = cudaGetErrorString(e);
             return GBFFT_ERR_CUDA;
         }
-        p.prepared = true;
     }
     if (!p.h_error) {
         if (cudaHostAlloc(&p.h_error, sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) {
@@ -542,7 +556,7 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
         }
         *p.h_error = 0;
     }
-    if (p.tw.ptr == nullptr && p.tw_entries > 0) {
+    if (fill && p.tw_entries > 0) {
         int st = p.tw.ensure(p.tw_entries * sizeof(float2), why);
         if (st != GBFFT_OK) return st;
         for (size_t s = 0; s < p.segs.size(); s += 16) {
@@ -554,11 +568,11 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
             }
         }
     }
-    if (pipe && !p.fact.ptr) {
+    if (fill_fact) {
         std::string no_room;
         cudaError_t e = ragged_pipe_prepare();
         if (p.fact.ensure(p.fact_entries * sizeof(float4), no_room) != GBFFT_OK) {
-            p.pipe = pipe = false;  // the barrier form needs no factor table
+            p.pipe = fill_fact = pipe = false;  // the barrier form needs no factor table
         } else {
             const float2 *tw = (const float2 *)p.tw.ptr;
             for (int L = 14; L <= kRagMaxLogN && e == cudaSuccess; ++L) {
@@ -605,6 +619,8 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
         why = cudaGetErrorString(e);
         return GBFFT_ERR_CUDA;
     }
+    p.filled = true;
+    p.fact_filled |= fill_fact;
     p.dirty[pipe] = false;
     return GBFFT_OK;
 }
