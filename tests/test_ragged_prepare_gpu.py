@@ -1,4 +1,6 @@
-"""GPU: what a ragged plan keeps between calls is complete or not there."""
+"""GPU: what a ragged plan keeps between calls -- tables and queues -- is complete or not
+there: after a first call under capture, and whichever of the two forms (ring of tiles,
+barrier) the calls before took."""
 import numpy as np
 import pytest
 
@@ -71,3 +73,28 @@ def test_tables_after_a_first_call_under_capture(lib_built, prec, large):
             plan.wait()
             _check(torch, x, y, descs)
         plan.close()
+
+
+@pytest.mark.parametrize("first,then", [(0, 8), (8, 0)])
+def test_one_ordinary_call_prepares_both_forms(gpu_ctx, first, then):
+    """A call on 16-byte boundaries takes the ring, one 8 bytes on the barrier form; either
+    makes ready what the other needs under capture."""
+    torch = pytest.importorskip("torch")
+    descs, total = _large()
+    x, y = _data(torch, total + 1)
+    xa, ya = x[1:].clone(), torch.full_like(x[1:], float("nan"))
+    buf = {0: (xa.data_ptr(), ya.data_ptr()), 8: (x.data_ptr() + 8, y.data_ptr() + 8)}
+    plan = gpu_ctx.ragged_plan(descs)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    plan.execute(*buf[first], total, use_graph=False, stream=stream.cuda_stream)
+    plan.wait(stream.cuda_stream)
+    with torch.cuda.graph(graph, stream=stream):
+        plan.execute(*buf[then], total, use_graph=False, stream=stream.cuda_stream)
+    for _ in range(2):
+        y.fill_(float("nan"))
+        ya.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        _check(torch, xa, ya if then == 0 else y[1:], descs)
+    plan.close()

@@ -32,6 +32,7 @@
 // rag_pipe_pays below has the rule).
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -277,7 +278,7 @@ struct RaggedPlanImpl {
     uint32_t spin_limit = 1u << 22;
     bool drop_producers = false;
     uint32_t lag_per_sm = 4;  // GBFFT_RAGGED_OPT_LAG
-    bool dirty[2] = {true, true};  // [barrier, warp-column form]: its queue must be (re)uploaded
+    bool dirty = true;        // the queues must be (re)uploaded
     std::vector<RagXform> xf;
     std::vector<RagItem> items;
     std::vector<uint32_t> order;
@@ -299,9 +300,9 @@ struct RaggedPlanImpl {
     cudaStream_t capture_stream = nullptr;
     uint64_t launches = 0;
     int sms = 0;
-    // Tables that a launch may read.  Set when the stream that filled them has been waited
-    // for: an allocated table may be a failed call's, or its fill may have gone into a capture.
-    bool filled = false, fact_filled = false;
+    // The tables may be read.  Set when the stream that filled them has been waited for:
+    // an allocated table may be a failed call's, or its fill may have gone into a capture.
+    bool filled = false;
     int precision = GBFFT_PREC_FP32;
     void *gtab = nullptr;   // split form: the G operand parts (fft_passes_tc.cu)
     // Warp-column form (fft_ragged_pipe.cu), taken out of place on 16-byte
@@ -419,7 +420,7 @@ static void build_items(RaggedPlanImpl &p) {
     if (p.pipe) queue_items(p, rows, two, total_p1, p.lag_set ? p.lag_per_sm : kRagPipeLag, p.pipe_items);
     if (p.order.empty()) p.order.push_back(0);
     p.nitems = (uint32_t)p.items.size();
-    p.dirty[0] = p.dirty[1] = true;
+    p.dirty = true;
 }
 
 int ragged_plan_build(RaggedPlanImpl *&out, int device, const gbfft_ragged_desc *descs, uint32_t count,
@@ -527,13 +528,14 @@ static bool capturing(cudaStream_t stream) {
     return false;
 }
 
-// Makes the tables and copies the queue that a launch of this form takes.  `pipe` is
-// cleared where the warp-column form's tables find no room.
-static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cudaStream_t stream, std::string &why) {
+// Makes the tables and copies the queues that the plan's launches take, of both forms
+// whichever this call runs: a later call may be under capture, where neither can be made.
+// (1250 transforms of 2^8..2^18, create and first execute: 630 us, against 637 with one
+// form's queue and a zeroed staging block.)
+static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, cudaStream_t stream, std::string &why) {
     const bool fill = !p.filled;
-    bool fill_fact = pipe && !p.fact_filled;
-    if ((fill || fill_fact || p.dirty[pipe]) && capturing(stream)) {
-        why = "a ragged plan's first call fills its tables and cannot be captured";
+    if ((fill || p.dirty) && capturing(stream)) {
+        why = "a ragged plan's first call makes its tables and cannot be captured";
         return GBFFT_ERR_CUDA;
     }
     if (fill) {
@@ -568,11 +570,11 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
             }
         }
     }
-    if (fill_fact) {
+    if (fill && p.pipe) {
         std::string no_room;
         cudaError_t e = ragged_pipe_prepare();
         if (p.fact.ensure(p.fact_entries * sizeof(float4), no_room) != GBFFT_OK) {
-            p.pipe = fill_fact = pipe = false;  // the barrier form needs no factor table
+            p.pipe = false;  // the barrier form needs no factor table
         } else {
             const float2 *tw = (const float2 *)p.tw.ptr;
             for (int L = 14; L <= kRagMaxLogN && e == cudaSuccess; ++L) {
@@ -591,13 +593,12 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
         int st = p.ws.ensure(p.ws_samples * sizeof(float2), why);
         if (st != GBFFT_OK) return st;
     }
-    // [barrier form's queue | transforms | order | warp-column form's queue | counters]:
-    // each form takes the part that it needs in one copy, at its first launch
-    if (!p.dirty[pipe]) return GBFFT_OK;
+    if (!p.dirty) return GBFFT_OK;
+    // [barrier form's queue | transforms | order | warp-column form's queue | counters]
     const size_t xf_bytes = p.xf.size() * sizeof(RagXform);
     const size_t it_bytes = p.items.size() * sizeof(RagItem);
     const size_t or_bytes = p.order.size() * sizeof(uint32_t);
-    const size_t pi_bytes = p.pipe_items.size() * sizeof(RagItem);
+    const size_t pi_bytes = p.pipe ? p.pipe_items.size() * sizeof(RagItem) : 0;
     p.off_xf = (it_bytes + 255) & ~(size_t)255;
     p.off_order = (p.off_xf + xf_bytes + 255) & ~(size_t)255;
     p.off_pitems = (p.off_order + or_bytes + 255) & ~(size_t)255;
@@ -605,13 +606,12 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
     p.counters_bytes = (3 + (size_t)p.count) * sizeof(uint32_t);
     int st = p.meta.ensure(p.off_counters + p.counters_bytes, why);
     if (st != GBFFT_OK) return st;
-    const size_t from = pipe ? p.off_xf : 0, to = pipe ? p.off_counters : p.off_pitems;
-    std::vector<char> host(to - from, 0);
-    if (xf_bytes) memcpy(host.data() + (p.off_xf - from), p.xf.data(), xf_bytes);
-    memcpy(host.data() + (p.off_order - from), p.order.data(), or_bytes);
-    if (!pipe && it_bytes) memcpy(host.data(), p.items.data(), it_bytes);
-    if (pipe) memcpy(host.data() + (p.off_pitems - from), p.pipe_items.data(), pi_bytes);
-    cudaError_t e = cudaMemcpyAsync((char *)p.meta.ptr + from, host.data(), host.size(), cudaMemcpyHostToDevice, stream);
+    std::unique_ptr<char[]> host(new char[p.off_counters]);  // (the gaps are never read)
+    if (it_bytes) memcpy(host.get(), p.items.data(), it_bytes);
+    if (xf_bytes) memcpy(host.get() + p.off_xf, p.xf.data(), xf_bytes);
+    memcpy(host.get() + p.off_order, p.order.data(), or_bytes);
+    if (pi_bytes) memcpy(host.get() + p.off_pitems, p.pipe_items.data(), pi_bytes);
+    cudaError_t e = cudaMemcpyAsync(p.meta.ptr, host.get(), p.off_counters, cudaMemcpyHostToDevice, stream);
     // (from then on every launch leaves them zero)
     if (e == cudaSuccess) e = cudaMemsetAsync((char *)p.meta.ptr + p.off_counters, 0, p.counters_bytes, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
@@ -620,8 +620,7 @@ static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, bool &pipe, cuda
         return GBFFT_ERR_CUDA;
     }
     p.filled = true;
-    p.fact_filled |= fill_fact;
-    p.dirty[pipe] = false;
+    p.dirty = false;
     return GBFFT_OK;
 }
 
@@ -684,9 +683,10 @@ static cudaError_t rag_enqueue(RaggedPlanImpl &p, const void *in, void *out, boo
 
 int ragged_plan_execute(RaggedPlanImpl &p, const void *in, void *out, cudaStream_t stream, bool use_graph,
                         std::string &why) {
-    bool pipe = p.pipe && in != (const void *)out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && tensor_map_encoder();
-    int st = ragged_plan_upload(p, in == (const void *)out, pipe, stream, why);
+    int st = ragged_plan_upload(p, in == (const void *)out, stream, why);
     if (st != GBFFT_OK) return st;
+    const bool pipe =
+        p.pipe && in != (const void *)out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && tensor_map_encoder();
     cudaError_t e;
     if (!use_graph) {
         e = rag_enqueue(p, in, out, pipe, stream);
