@@ -184,7 +184,7 @@ int gbfft_ragged_execute(gbfft_ragged_plan *plan, const void *d_in, void *d_out,
                          int use_graph, void *stream);
 
 /* Synchronise `stream` and report GBFFT_ERR_TIMEOUT if a dependency wait of
- * the last execution gave up. */
+ * any execution since the last call of this gave up. */
 int gbfft_ragged_wait(gbfft_ragged_plan *plan, void *stream);
 
 /* Number of kernel launches issued by the plan so far. */

@@ -1,6 +1,6 @@
 """GPU: what a ragged plan keeps between calls -- tables and queues -- is complete or not
 there: after a first call under capture, and whichever of the two forms (ring of tiles,
-barrier) the calls before took."""
+barrier) the calls before took.  A time-out stays reported until it is read."""
 import numpy as np
 import pytest
 
@@ -97,4 +97,27 @@ def test_one_ordinary_call_prepares_both_forms(gpu_ctx, first, then):
         graph.replay()
         torch.cuda.synchronize()
         _check(torch, xa, ya if then == 0 else y[1:], descs)
+    plan.close()
+
+
+@pytest.mark.parametrize("large", [False, True])
+def test_a_time_out_is_reported_by_the_next_wait(gpu_ctx, large):
+    """A run that gave up, then a good one with no wait between: the wait reports the first."""
+    import gbfft
+    torch = pytest.importorskip("torch")
+    descs, total = _large() if large else _small()
+    x, y = _data(torch, total)
+    plan = gpu_ctx.ragged_plan(descs)
+    plan.set(gbfft.RAGGED_OPT_SPIN_LIMIT, 2000)
+    plan.set(gbfft.RAGGED_OPT_TEST_DROP_PRODUCERS, 1)
+    plan.execute(x, y, total, use_graph=False)
+    plan.set(gbfft.RAGGED_OPT_TEST_DROP_PRODUCERS, 0)
+    plan.set(gbfft.RAGGED_OPT_SPIN_LIMIT, 1 << 22)
+    plan.execute(x, y, total, use_graph=False)
+    with pytest.raises(gbfft.GbfftError) as e:
+        plan.wait()
+    assert e.value.status == gbfft.ERR_TIMEOUT
+    _check(torch, x, y, descs)
+    plan.execute(x, y, total, use_graph=True)
+    plan.wait()  # reported once
     plan.close()

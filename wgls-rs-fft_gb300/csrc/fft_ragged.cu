@@ -291,7 +291,7 @@ struct RaggedPlanImpl {
     DeviceBuffer meta;        // xf | items | order | counters
     DeviceBuffer tw;
     DeviceBuffer ws;
-    uint32_t *h_error = nullptr;  // pinned copy of the error flag
+    uint32_t *h_error = nullptr;  // pinned word that a launch which gave up sets
     size_t off_xf = 0, off_order = 0, off_counters = 0, counters_bytes = 0;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;

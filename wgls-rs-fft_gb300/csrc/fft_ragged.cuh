@@ -42,7 +42,7 @@ struct RagParams {
     uint32_t *done1;
     uint32_t *error;
     uint32_t *exits;        // CTAs that have left
-    uint32_t *host_error;   // pinned host word: the launch's error flag, written by the last CTA
+    uint32_t *host_error;   // pinned host word: set by the last CTA of a launch that gave up; the host clears it
     uint32_t counters;      // words from item_counter on: zero before and after a launch
     const float2 *sub[16];   // sub-pass tables of a length-2^L in-SMEM FFT
     const float2 *lo[kRagMaxLogN + 1];
@@ -75,7 +75,8 @@ __device__ __forceinline__ void rag_finish(const RagParams &P, int *flag) {
     __syncthreads();
     if (!*flag) return;
     __threadfence();
-    if (threadIdx.x == 0) *(volatile uint32_t *)P.host_error = *(volatile uint32_t *)P.error;
+    // (set only: a good launch after it must not take an unread report back)
+    if (threadIdx.x == 0 && *(volatile uint32_t *)P.error != 0u) *(volatile uint32_t *)P.host_error = 1u;
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < P.counters; i += THREADS) P.item_counter[i] = 0u;
 }
