@@ -521,20 +521,13 @@ int ragged_plan_build(RaggedPlanImpl *&out, int device, const gbfft_ragged_desc 
     return GBFFT_OK;
 }
 
-static bool capturing(cudaStream_t stream) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
-    cudaGetLastError();
-    return false;
-}
-
 // Makes the tables and copies the queues that the plan's launches take, of both forms
 // whichever this call runs: a later call may be under capture, where neither can be made.
 // (1250 transforms of 2^8..2^18, create and first execute: 630 us, against 637 with one
 // form's queue and a zeroed staging block.)
 static int ragged_plan_upload(RaggedPlanImpl &p, bool in_place, cudaStream_t stream, std::string &why) {
     const bool fill = !p.filled;
-    if ((fill || p.dirty) && capturing(stream)) {
+    if ((fill || p.dirty) && stream_capturing(stream)) {
         why = "a ragged plan's first call makes its tables and cannot be captured";
         return GBFFT_ERR_CUDA;
     }

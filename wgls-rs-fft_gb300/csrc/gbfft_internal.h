@@ -52,6 +52,15 @@ struct RowsKernelInfo {
     int nseg = 0;
     int tw_entries = 0;
 };
+// Whether work on the stream goes into a capture, where nothing can be allocated or
+// waited for (an unanswered question counts as yes).
+inline bool stream_capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 // A kernel that begins with stream_order(), brought up while the launch before it in
 // the stream still runs; it touches no memory before that one is complete (twiddle.cu).
 cudaError_t launch_overlapped(const void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t stream);

@@ -417,7 +417,18 @@ int plan_execute(const Plan &p, const float2 *in, float2 *out, uint64_t batch, i
     const bool pair2 = p.has_fused && p.passes.size() == 2 && (const void *)in != (const void *)out;
     const uint64_t ngroups = batch * fd.groups_per_transform;
     if ((pair2 || pair3 || wide) && ctr && ngroups <= 0x7fffffffull) {
-        const size_t want = (2 + (size_t)ngroups) * sizeof(uint32_t);
+        size_t want = (2 + (size_t)ngroups) * sizeof(uint32_t);
+        if (wide) {
+            // A later call of this size and batch that needs the three passes may be under
+            // capture, where neither their counters nor their workspace can be made.
+            const size_t want3 = (2 + (size_t)batch * p.fused.groups_per_transform) * sizeof(uint32_t);
+            const size_t ws_bytes = ((size_t)batch << p.logn) * sizeof(float2);
+            if ((ctr->bytes < want3 || ws.bytes < ws_bytes) && !stream_capturing(stream)) {
+                want = std::max(want, want3);
+                std::string no_room;  // (no room: this launch needs no workspace)
+                (void)ws.ensure(ws_bytes, no_room);
+            }
+        }
         if (ctr->bytes < want) {
             int st = ctr->ensure(want, why);
             if (st != GBFFT_OK) return st;
