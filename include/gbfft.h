@@ -109,12 +109,13 @@ int gbfft_c2c_host_rows(gbfft_ctx *ctx, const float *const *in_rows,
 
 /* Device-resident entry point (new; no reference counterpart -- the reference
  * always round-trips through host memory).  `d_in`/`d_out` are device
- * pointers to batch*n interleaved complex<f32>; they may alias and need only
- * the alignment of complex<f32> (8 bytes: every kernel reads and writes
- * caller memory one sample at a time; wider accesses touch only the
- * library's own buffers).  Work is
- * enqueued on `stream` (a cudaStream_t; NULL is the CUDA default stream, as
- * everywhere in CUDA) and the call returns without synchronising. */
+ * pointers to batch*n interleaved complex<f32>, the same buffer or disjoint
+ * ones (a partial overlap gives the transform of the input for 2^21 <= N <=
+ * 2^26 only, whose first pass then writes to a workspace).  They need only the
+ * alignment of complex<f32> (8 bytes); out of place on 16-byte boundaries,
+ * the faster tiled copies serve N = 2^15..2^26.  Work is enqueued on
+ * `stream` (a cudaStream_t; NULL is the CUDA default stream, as everywhere in
+ * CUDA) and the call returns without synchronising. */
 int gbfft_c2c_device(gbfft_ctx *ctx, const void *d_in, void *d_out, uint64_t n,
                      uint64_t batch, int direction, void *stream);
 

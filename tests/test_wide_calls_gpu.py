@@ -1,5 +1,6 @@
 """GPU: 2^21 and 2^22, which take one two-pass launch where the buffers allow it, in the
-calls that cannot, under capture after an ordinary call that could."""
+calls that cannot: under capture after an ordinary call that could, and with an output
+that overlaps the input."""
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -48,3 +49,21 @@ def test_capture_after_one_ordinary_call(lib_built, logn, form):
         torch.cuda.synchronize()
         got = {"in place": a, "8 bytes on": out[1:], "noise": y}[form]
         assert _rel(torch, got, want.to(torch.complex128)) <= TOL_REL_L2
+
+
+@pytest.mark.parametrize("logn", [21, 22])
+@pytest.mark.parametrize("shift", [2, 4096, -4096, (1 << 21) + 2, -(1 << 21) - 2])
+def test_output_that_overlaps_the_input(lib_built, logn, shift):
+    """Samples apart by `shift`: the three-pass form reads all of the input before it writes
+    any of the output."""
+    import gbfft
+    torch = pytest.importorskip("torch")
+    n, batch = 1 << logn, 3
+    buf = torch.view_as_complex(torch.randn(batch * n + abs(shift), 2, device="cuda"))
+    i, o = (0, shift) if shift > 0 else (-shift, 0)
+    x, y = buf[i:i + batch * n], buf[o:o + batch * n]
+    want = torch.fft.ifft(x.view(batch, n).to(torch.complex128)).view(-1)
+    with gbfft.Context(0) as ctx:
+        ctx.c2c_device(x, y, n, batch, gbfft.INVERSE, stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+    assert _rel(torch, y, want) <= TOL_REL_L2

@@ -51,9 +51,12 @@ int pass_sub_segments(int logr, int loge, TwiddleSegment *out, uint64_t base, in
     }
 }
 
-bool wide_usable(const float2 *in, const float2 *out, const LoadOps &ops) {
-    return in != out && (((uintptr_t)in | (uintptr_t)out) & 15u) == 0 && !ops.win && ops.noise_sigma == 0.f &&
-           tensor_map_encoder() != nullptr;
+// Disjoint: the launch writes outputs while it still reads inputs, which the first of
+// three passes has copied out of the way of an output that overlaps them.
+bool wide_usable(const float2 *in, const float2 *out, uint64_t samples, const LoadOps &ops) {
+    const uintptr_t a = (uintptr_t)in, b = (uintptr_t)out;
+    return (a > b ? a - b : b - a) >= samples * sizeof(float2) && ((a | b) & 15u) == 0 && !ops.win &&
+           ops.noise_sigma == 0.f && tensor_map_encoder() != nullptr;
 }
 
 cudaError_t fused_prepare(FusedDesc &d) {

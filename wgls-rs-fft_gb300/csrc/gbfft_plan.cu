@@ -411,7 +411,7 @@ int plan_execute(const Plan &p, const float2 *in, float2 *out, uint64_t batch, i
     // Fused pass pair: both passes of a two-pass transform (out of place
     // only: its first pass writes into `out` while other tiles still read
     // `in`), or the last two of three after the first pass into the workspace.
-    const bool wide = p.has_wide && ctr && wide_usable(in, out, ops) && batch <= 0x7fffffffull;
+    const bool wide = p.has_wide && ctr && wide_usable(in, out, batch << p.logn, ops) && batch <= 0x7fffffffull;
     const FusedDesc &fd = wide ? p.wide : p.fused;
     const bool pair3 = p.has_fused && p.passes.size() == 3 && !wide;
     const bool pair2 = p.has_fused && p.passes.size() == 2 && (const void *)in != (const void *)out;
@@ -447,7 +447,7 @@ int plan_execute(const Plan &p, const float2 *in, float2 *out, uint64_t batch, i
             if (st != GBFFT_OK) return st;
             const PassDesc &d0 = p.passes[0];
             // (its counters, one a 2^20 samples, are no more than the pair's: one a 2^20)
-            if (p.has_lone && wide_usable(in, (const float2 *)ws.ptr, ops)) {
+            if (p.has_lone && wide_usable(in, (const float2 *)ws.ptr, batch << p.logn, ops)) {
                 e = cudaSuccess;
                 for (uint64_t b = 0; b < batch && e == cudaSuccess; ++b)
                     e = pipe_first_launch(p.lone, in + (b << p.logn), (float2 *)ws.ptr + (b << p.logn), p.logn,

@@ -192,8 +192,8 @@ bool pipe2_kernel_info(int logr1, int logr2, PipeDesc &d, int loge);
 bool pipe3_kernel_info(int logn, PipeDesc &d);
 // N = 2^21, 2^22 as two passes of radix 2^11 and 2^(logn - 11)
 bool pipe_wide_info(int logn, FusedDesc &d);
-// Whether buffers and options suit that launch.
-bool wide_usable(const float2 *in, const float2 *out, const LoadOps &ops);
+// Whether buffers (of `samples` each) and options suit that launch.
+bool wide_usable(const float2 *in, const float2 *out, uint64_t samples, const LoadOps &ops);
 // inflight: tiles that the launch's CTAs hold at once
 uint32_t fused_lag(uint64_t inflight, uint32_t tiles_per_group, uint64_t group_samples, uint64_t ngroups);
 cudaError_t pipe_first_launch(const FusedDesc &d, const float2 *in, float2 *out, int logn, const float2 *tw_a,

@@ -168,7 +168,7 @@ impl GpuFft {
     }
 
     /// Device-resident transform: `d_in` / `d_out` are device pointers to
-    /// `batch * n` interleaved complex<f32> (8-byte aligned; they may alias),
+    /// `batch * n` interleaved complex<f32> (8-byte aligned; the same buffer or disjoint ones),
     /// enqueued on `stream` (a cudaStream_t, null for the default stream).
     ///
     /// # Safety
