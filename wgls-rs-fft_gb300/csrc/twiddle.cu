@@ -121,11 +121,7 @@ cudaError_t hann_fill(float *w, uint64_t n, cudaStream_t stream) {
 // 229.8.  Into a capture goes an ordinary launch: the graph has edges of its own (and
 // starts its nodes 2 us apart), and the node fits whatever body it is put into.
 cudaError_t launch_overlapped(const void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t stream) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return cudaLaunchKernel(fn, grid, block, args, smem, stream);
-    }
+    if (stream_capturing(stream)) return cudaLaunchKernel(fn, grid, block, args, smem, stream);
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
