@@ -1,8 +1,9 @@
 """ctypes binding of the C ABI in include/gbfft.h.
 
 Context.c2c_device, the call whose own cost shows, goes through a small extension module
-(``_call.c``) where that is built.  There is no fallback for the library: if libgbfft.so is missing or cannot be loaded, every
-entry point raises.  The library is the only implementation of the transform.
+(``_call.c``) where that is built and loads.  There is no fallback for the library: if
+libgbfft.so is missing or cannot be loaded, every entry point raises.  The library is the
+only implementation of the transform.
 """
 from __future__ import annotations
 
@@ -84,6 +85,19 @@ def lib_path() -> str:
     return os.environ.get("GBFFT_LIB", LIB_PATH)
 
 
+def _load_call():
+    """c2c of the extension module, or None where it is not built or does not load here."""
+    if not os.path.exists(CALL_PATH):
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_gbfft_call", CALL_PATH)
+    try:
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_gbfft_call", loader))
+        loader.exec_module(module)
+    except ImportError:
+        return None
+    return module.c2c
+
+
 def load():
     """Load libgbfft.so (raises if it is absent -- there is no CPU path)."""
     global _lib, _c2c
@@ -97,12 +111,7 @@ def load():
                 f = getattr(L, name)
                 f.restype = res
                 f.argtypes = args
-            if os.path.exists(CALL_PATH):
-                loader = importlib.machinery.ExtensionFileLoader("_gbfft_call", CALL_PATH)
-                spec = importlib.util.spec_from_loader("_gbfft_call", loader)
-                module = importlib.util.module_from_spec(spec)
-                loader.exec_module(module)
-                _c2c = module.c2c
+            _c2c = _load_call()
             _lib = L
         return _lib
 
