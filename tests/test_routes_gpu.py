@@ -122,3 +122,23 @@ def test_ragged(gpu_ctx, stream):
             assert len(names) == 1 and ("fft_ragged_pipe_kernel" in names[0]) == ring, (count, offset, names)
             assert ring or "fft_ragged_kernel" in names[0], names
         plan.close()
+
+
+@pytest.mark.parametrize("logn,prec,loop", [(8, 1, True), (12, 1, False), (12, 4, True), (13, 3, True), (13, 4, True), (14, 1, True),
+                                            (14, 2, True), (14, 4, False)])
+def test_split_single_pass_loop(lib_built, stream, logn, prec, loop):
+    """A large launch takes the tile loop where that is the faster one (fft_rows_tc.cuh)."""
+    import gbfft
+    torch = pytest.importorskip("torch")
+    n, batch = 1 << logn, (1 << 24) >> logn
+    x = torch.zeros((n * batch, 2), device="cuda")
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    with gbfft.Context(0) as ctx:
+        ctx.set_precision(prec)
+        args = (x, y, n, batch, gbfft.FORWARD)
+        ctx.c2c_device(*args, stream=stream.cuda_stream)
+        torch.cuda.synchronize()
+        names = _kernels(ctx._L, stream, lambda: ctx.c2c_device(*args, stream=stream.cuda_stream))
+    assert len(names) == 1 and "fft_rows_tc_kernel" in names[0]
+    assert ("Lb1E" in names[0]) == loop, names

@@ -58,8 +58,9 @@ struct RowsTcCfg {
     static_assert(MINB >= 1 && MINB * TMEM_COLS <= 512, "tensor memory of an SM");
     // Where the loop is built: not for the 16-bit kinds at 2^12 and 2^13, whose one-shot
     // tiles are as large and as many an SM (2^13 FP16, 2048 transforms: 102.4 us one-shot,
-    // 108.8 looped in 6.7 rounds; 8192: 393, 383)
-    static constexpr bool HAS_LOOP = Gm::PARTS == 3 || Gm::ELEM == 4 || LOGN < 12 || LOGN == 14;
+    // 108.8 looped in 6.7 rounds; 8192: 393, 383), nor for BF16 x 6 at 2^14 (2896 transforms:
+    // 467.6, 480.4; 588: 95.6, 100.2)
+    static constexpr bool HAS_LOOP = LOGN < 12 || Gm::ELEM == 4 || (Gm::PARTS == 3 ? LOGN < 14 : LOGN == 14);
 };
 
 template <int LOGN, int DIRC, int KIND, bool LOOP>
