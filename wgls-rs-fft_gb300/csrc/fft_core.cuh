@@ -280,10 +280,14 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
 // stream_wait: wait for the launches before it in the stream.  The next launch is
 // brought up as this one's CTAs leave.
 // stream_order: that, and let the next launch be brought up at once -- in this order, so
-// that whatever is brought up has only this launch left to wait for.  For the
-// single-pass kernels (split form, 2^8 x 64 FP16: 4.64 us against 4.79, 2^13 x 8 TF32 12.5
-// against 12.8); the pairs run their last tiles beside CTAs that wait, and lose (2^24 x 4:
-// 473 us against 428, 2^16 x 1024 FP16 480 against 477).
+// that whatever is brought up has only this launch left to wait for.  For the split
+// single-pass kernels, whose start is long (2^8 x 64 FP16: 4.64 us against 4.79, 2^8 x 2048
+// BF16 x 6 6.14 against 6.36).  The others lose: CTAs that wait take the room that this
+// launch's own later CTAs want.  The FP32 single pass gains at most 0.1 us (2^13 x 32 4.65
+// against 4.72) and loses up to 5 between half a wave and three, to below an ordinary
+// launch (2^6 x 20171: 6.60 us with it, 4.42 without, 6.19 in an ordinary launch; 2^5 x
+// 40342 10.8, 8.2, 10.3; 2^4 x 80684 18.5, 13.5, 16.5; 2^14 x 256 20.6, 18.6, 20.6); the
+// pairs 2^24 x 4 473 us against 428, 2^16 x 1024 FP16 480 against 477.
 __device__ __forceinline__ void stream_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void stream_order() {
     stream_wait();

@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(RowsCfg<LOGN, LOGS, LE>::THREADS, RowsCfg<LOGN
 fft_rows_persistent_kernel(const float2 *in, float2 *out, uint64_t batch, const float2 *__restrict__ tw,
                            float in_im_sign, float out_re_scale, float out_im_scale, LoadOps ops,
                            const uint64_t *, const uint64_t *) {  // (no row tables: the host never passes them)
-    stream_order();
+    stream_wait();
     using C = RowsCfg<LOGN, LOGS, LE>;
     extern __shared__ float2 smem_rows[];
     constexpr uint32_t kTileSamples = C::G * C::N;

@@ -37,10 +37,7 @@ __global__ void __launch_bounds__(RowsCfg<LOGN, LOGS, LE>::THREADS, RowsCfg<LOGN
 fft_rows_kernel(const float2 *in, float2 *out, uint64_t batch, const float2 *__restrict__ tw,
                 float in_im_sign, float out_re_scale, float out_im_scale, LoadOps ops,
                 const uint64_t *__restrict__ tab_in, const uint64_t *__restrict__ tab_out) {
-    // (N = 1 is 2 KB a CTA, bound by the rate of CTAs, which the second instruction slows:
-    // 2^24 transforms 67.6 us with it, 52.0 without, 53.6 in an ordinary launch; no other size)
-    if constexpr (LOGN > 0) stream_order();
-    else stream_wait();
+    stream_wait();
     using C = RowsCfg<LOGN, LOGS, LE>;
     extern __shared__ float2 smem_rows[];
     auto ref = [&](int g) {

@@ -61,8 +61,9 @@ inline bool stream_capturing(cudaStream_t stream) {
     return true;
 }
 
-// A kernel that begins with stream_order(), brought up while the launch before it in
-// the stream still runs; it touches no memory before that one is complete (twiddle.cu).
+// A kernel that waits for the launches before it (stream_wait, stream_order: fft_core.cuh),
+// brought up while the one before still runs or as its CTAs leave (twiddle.cu).  Until that
+// wait it touches nothing that a launch writes: it may read a plan's tables.
 cudaError_t launch_overlapped(const void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t stream);
 
 // logs: log2 of the samples a CTA moves (12; 11 or 13 for N = 2^6 .. 2^11);
