@@ -776,6 +776,9 @@ int ragged_plan_set(RaggedPlanImpl &p, int option, uint64_t value, std::string &
 
 void ragged_plan_free(RaggedPlanImpl *p) {
     if (!p) return;
+    // Waits for launches in flight, whose last CTA may still write the host word (pinned
+    // memory is not promised to wait).
+    p->meta.release();
     if (p->graph_exec) cudaGraphExecDestroy(p->graph_exec);
     if (p->graph) cudaGraphDestroy(p->graph);
     if (p->capture_stream) cudaStreamDestroy(p->capture_stream);
