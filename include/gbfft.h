@@ -113,9 +113,13 @@ int gbfft_c2c_host_rows(gbfft_ctx *ctx, const float *const *in_rows,
  * ones (a partial overlap gives the transform of the input for 2^21 <= N <=
  * 2^26 only, whose first pass then writes to a workspace).  They need only the
  * alignment of complex<f32> (8 bytes); out of place on 16-byte boundaries,
- * the faster tiled copies serve N = 2^15..2^26.  Work is enqueued on
- * `stream` (a cudaStream_t; NULL is the CUDA default stream, as everywhere in
- * CUDA) and the call returns without synchronising. */
+ * the faster tiled copies serve N = 2^15..2^26.  Placement and alignment do
+ * not change the result's bits but at two places: N = 2^17..2^20 in place
+ * (other sub-pass radices), and N = 2^21 and 2^22, which are two passes out of
+ * place on 16-byte boundaries without load options and three otherwise.
+ * Every form stays below 2e-7 relative L2 error there.  Work is
+ * enqueued on `stream` (a cudaStream_t; NULL is the CUDA default stream, as
+ * everywhere in CUDA) and the call returns without synchronising. */
 int gbfft_c2c_device(gbfft_ctx *ctx, const void *d_in, void *d_out, uint64_t n,
                      uint64_t batch, int direction, void *stream);
 
@@ -138,8 +142,8 @@ int gbfft_c2c_device(gbfft_ctx *ctx, const void *d_in, void *d_out, uint64_t n,
  * cudaDeviceReset, so do not call this entry on a device after resetting it.
  * All calls on a device share the one scratch array, so calls that overlap on
  * the GPU race: serialise them.  It runs the plain two-pass schedule (one
- * launch per pass), 10-15 % slower at these sizes than gbfft_c2c_device's
- * fused pass pair. */
+ * launch per pass): 0.5 to 1.0 of gbfft_c2c_device's time up to 2^20 samples
+ * a call, 0.9 to 1.35 of it at 2^22. */
 int gbfft_c2c_device_noalloc(const void *d_in, void *d_out, uint64_t n,
                              uint64_t batch, int direction, void *stream);
 
@@ -178,9 +182,14 @@ int gbfft_ragged_plan_set(gbfft_ragged_plan *plan, int option, uint64_t value);
 /* Enqueue the plan on `stream` (NULL = default stream).  `capacity` is the
  * size of d_in and of d_out in complex samples; a descriptor reaching past it
  * is rejected (GBFFT_ERR_INVALID_ARGUMENT) before anything is launched.  With
- * use_graph != 0 the reset + launch sequence is captured once into a CUDA
- * graph (per (d_in, d_out) pair) and replayed.  Asynchronous: call
- * gbfft_ragged_wait. */
+ * use_graph != 0 the launch (one kernel) is captured once into a CUDA graph
+ * (per (d_in, d_out) pair) and replayed.  The first call of a plan, and of an
+ * option set since, makes tables and synchronises `stream`, and is refused on
+ * a stream under capture; the first call in place allocates a workspace, and
+ * cannot be captured either.
+ * Large FP32 sets run in another form out of place on 16-byte boundaries than
+ * elsewhere: the bits of their two-pass transforms then differ (1.7e-7
+ * relative L2 error either way).  Asynchronous: call gbfft_ragged_wait. */
 int gbfft_ragged_execute(gbfft_ragged_plan *plan, const void *d_in, void *d_out, uint64_t capacity,
                          int use_graph, void *stream);
 

@@ -281,8 +281,10 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
 // brought up as this one's CTAs leave.
 // stream_order: that, and let the next launch be brought up at once -- in this order, so
 // that whatever is brought up has only this launch left to wait for.  For the split
-// single-pass kernels, whose start is long (2^8 x 64 FP16: 4.64 us against 4.79, 2^8 x 2048
-// BF16 x 6 6.14 against 6.36).  The others lose: CTAs that wait take the room that this
+// single-pass kernels, whose start is long: 2 to 4 % on launches below half a wave (2^8 x 64
+// FP16 4.64 us against 4.79, 2^8 x 2048 BF16 x 6 6.14 against 6.36), against 3 to 12 % around
+// a wave (2^12 x 256 BF16 x 6 11.5 against 10.3, in an ordinary launch 12.4), nothing above
+// three.  The others lose: CTAs that wait take the room that this
 // launch's own later CTAs want.  The FP32 single pass gains at most 0.1 us (2^13 x 32 4.65
 // against 4.72) and loses up to 5 between half a wave and three, to below an ordinary
 // launch (2^6 x 20171: 6.60 us with it, 4.42 without, 6.19 in an ordinary launch; 2^5 x

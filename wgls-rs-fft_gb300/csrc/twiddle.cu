@@ -117,7 +117,7 @@ cudaError_t hann_fill(float *w, uint64_t n, cudaStream_t stream) {
 // programmatic launch the device brings the next grid up during the one before, and
 // stream_wait() holds it until that is complete: a pair of 2^10 x 9 transforms called
 // from C 8.2 -> 4.1 us (then the calls themselves), 2^16 x 32 21.0 -> 17.1, 2^18 x 1
-// 14.3 -> 11.3, 2^24 x 1 132 -> 120, 2^9 x 100003 119.6 -> 117.8, 2^16 x 1024 231.5 ->
+// 14.3 -> 11.3, 2^24 x 1 132 -> 120, 2^9 x 100003 119.5 -> 117.3, 2^16 x 1024 231.5 ->
 // 229.8.  Into a capture goes an ordinary launch: the graph has edges of its own (and
 // starts its nodes 2 us apart), and the node fits whatever body it is put into.
 cudaError_t launch_overlapped(const void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t stream) {
